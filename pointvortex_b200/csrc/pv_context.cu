@@ -22,6 +22,7 @@ using namespace pvb;
 namespace {
 
 thread_local std::string g_create_error;
+constexpr long double kPiLong = 3.14159265358979323846264338327950288L;
 
 // Butcher rows of the Dormand–Prince pair, src/timestep.h:8-15, and the weights b5, b4 of
 // src/timestep.cpp:69-73, as the reference's constant expressions evaluate them.
@@ -352,6 +353,21 @@ pv_status make_consts(const pv_params &p, GeometryConsts &g, std::string &messag
             g.k1 += 2.0 * u;
             g.k2 += 2.0 * u * u;
         }
+        if (p.image_layers >= kZetaMinLayers && lx >= kZetaMinLength && lx <= kZetaMaxLength) {
+            // z zeta(z) = P/Q in units of L/2, times L/pi, with a monic denominator
+            g.zeta = 1;
+            uint64_t bits;
+            std::memcpy(&bits, &g.half_lx, sizeof bits);
+            g.half_hi = static_cast<int>(bits >> 32);
+            const long double unit = 2.0L / lx, unit4 = unit * unit * unit * unit;
+            const long double lead = kZetaQ[3] * unit4 * unit4 * unit4;
+            long double power = 1.0L;
+            for (int k = 0; k < 6; ++k, power *= unit4) {
+                g.zp[k] = static_cast<double>(kZetaP[k] * power * (lx / kPiLong) / lead);
+                if (k < 3)
+                    g.zq[k] = static_cast<double>(kZetaQ[k] * power / lead);
+            }
+        }
         return PV_OK;
     }
     if (p.geometry == PV_GEOMETRY_DISK) {
@@ -588,8 +604,8 @@ pv_status ensure_state_capacity(pv_context *c, size_t n) {
         PV_CUDA(c, c->kx[s].ensure(np));
         PV_CUDA(c, c->ky[s].ensure(np));
     }
-    c->plan = plan_evaluation(c->gc.geometry, n, n, c->sm_count, 0, c->params.precision);
-    c->sym = plan_symmetric(n, c->sm_count, c->params.precision, c->gc.geometry);
+    c->plan = plan_evaluation(c->gc, n, n, c->sm_count, 0, c->params.precision);
+    c->sym = plan_symmetric(n, c->sm_count, c->params.precision, c->gc);
     if (near_field_used(c)) {
         const double r = near_radius_for(c, n);
         c->gc.near2 = r * r;
@@ -643,7 +659,7 @@ pv_status evaluate_host(pv_context *c, const double *x, const double *y, const d
         PV_CUDA(c, a->ensure(np));
     PV_CUDA(c, c->eu.ensure(padded(nt)));
     PV_CUDA(c, c->ev.ensure(padded(nt)));
-    const EvalPlan plan = plan_evaluation(c->gc.geometry, nt, n, c->sm_count, 0, c->params.precision);
+    const EvalPlan plan = plan_evaluation(c->gc, nt, n, c->sm_count, 0, c->params.precision);
     const size_t stride = padded(nt);
     PV_CUDA(c, c->epu.ensure(static_cast<size_t>(plan.num_chunks) * stride));
     PV_CUDA(c, c->epv.ensure(static_cast<size_t>(plan.num_chunks) * stride));

@@ -60,7 +60,7 @@ struct EvalPlan {
     size_t items() const { return static_cast<size_t>(num_chunks) * target_blocks; }
 };
 
-EvalPlan plan_evaluation(int geometry, size_t n_targets, size_t n_sources, int sm_count,
+EvalPlan plan_evaluation(const GeometryConsts &g, size_t n_targets, size_t n_sources, int sm_count,
                          int per_thread_override = 0, int precision = 0);
 // The autotuner's table of targets per thread (pv_set_tuning / pv_get_tuning).
 int tuning_lookup(int geometry, int precision, size_t n);
@@ -81,6 +81,7 @@ struct SymmetricPlan {
     int grid = 0;        // persistent CTAs
     int precision = 0;   // PV_PRECISION_FP64 or PV_PRECISION_FP32C
     int geometry = 0;    // GEO_PERIODIC or GEO_INFINITE
+    int zeta = 0;        // periodic FP64: the rational pair term (ZetaPair)
     int targets = 1;     // targets per lane off the diagonal (the plane: 4 or 8)
     int min_ctas = 0;    // periodic FP64: the kernel built for 7 or 8 CTAs per SM (0: default)
     int grid_ctas = 0;   // persistent CTAs per SM (grid / SMs)
@@ -92,7 +93,7 @@ constexpr size_t kSymmetricPlane32MinN = 16384; // the same for the FP32-compens
 constexpr size_t kSymmetricPlaneWideN = 32768;  // the plane from here: 8 targets per lane
 constexpr size_t kSymmetricPartialBytes = static_cast<size_t>(256) << 20;  // a grows past this
 constexpr size_t kSymmetricPartialBytesMax = static_cast<size_t>(4) << 30;  // beyond: ordered kernel
-SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, int geometry);
+SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const GeometryConsts &g);
 // The autotuner's table of the symmetric form (pv_set_symmetric_tuning); 0 = the built-in plan.
 int symmetric_tuning_lookup(int geometry, int precision, size_t n);
 // Autotuner table of the symmetric form's persistent grid: CTAs per SM (0: as many as fit), by

@@ -208,7 +208,7 @@ pv_status pv_evaluate_device_noalloc(const pv_params *params, const double *x, c
     // Split the sources into as many chunks as the plan wants and the scratch array can hold.
     const size_t np = padded_n(n);
     const size_t max_chunks = (kScratchDoubles - kControlDoubles - np) / (2 * np);
-    EvalPlan plan = plan_evaluation(g.geometry, n, n, sm_count);
+    EvalPlan plan = plan_evaluation(g, n, n, sm_count);
     if (static_cast<size_t>(plan.num_chunks) > max_chunks) {
         size_t chunk = (n + max_chunks - 1) / max_chunks;
         chunk = (chunk + 1) & ~static_cast<size_t>(1);

@@ -646,7 +646,8 @@ cudaError_t launch_rk4_steps(const Rk4Steps &p, int sm_count, cudaStream_t strea
     case GEO_INFINITE:
         return launch_rk4_steps_t<InfinitePair>(p, grid, stream);
     case GEO_PERIODIC:
-        return launch_rk4_steps_t<PeriodicPair>(p, grid, stream);
+        return p.stage[0].g.zeta ? launch_rk4_steps_t<ZetaPair>(p, grid, stream)
+                                 : launch_rk4_steps_t<PeriodicPair>(p, grid, stream);
     case GEO_DISK:
         return launch_rk4_steps_t<DiskPair>(p, grid, stream);
     default:

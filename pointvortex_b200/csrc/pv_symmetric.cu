@@ -62,8 +62,11 @@ __global__ void __launch_bounds__(kThreads, MINB)
                      const unsigned *__restrict__ items, unsigned n_items, unsigned *counter,
                      double2 *__restrict__ pr, size_t stride, GeometryConsts g) {
     extern __shared__ double2 reaction_smem[];
+    constexpr bool kBuffered = T <= 4;
+    __shared__ sym::SourceBuffer sources[kBuffered ? kThreads / 32 : 1];
     pdl_enter();
     const int lane = threadIdx.x & 31;
+    sym::SourceBuffer &src = sources[kBuffered ? threadIdx.x >> 5 : 0];
     double2 *reaction = reaction_smem + (threadIdx.x >> 5) * a * 32;  // this warp's sources
     const size_t block_len = static_cast<size_t>(32) * a;
     for (;;) {
@@ -81,7 +84,7 @@ __global__ void __launch_bounds__(kThreads, MINB)
         if (T > 1 && !diagonal) {
             for (int ib = 0; ib < a; ib += T) {
                 double tx[T], ty[T], tg[T], u[T], v[T];
-                bool t_ok[T], all_ok = true;
+                bool t_ok[T], all_ok = true, near = true;
 #pragma unroll
                 for (int t = 0; t < T; ++t) {
                     const size_t ti = I * block_len + static_cast<size_t>(ib + t) * 32 + lane;
@@ -90,6 +93,7 @@ __global__ void __launch_bounds__(kThreads, MINB)
                     tx[t] = t_ok[t] ? x[ti] : 0.0;
                     ty[t] = t_ok[t] ? y[ti] : 0.0;
                     tg[t] = t_ok[t] ? P::kScale * gs[ti] : 0.0;
+                    near = near && P::near(g, tx[t], ty[t]);
                     u[t] = 0.0;
                     v[t] = 0.0;
                 }
@@ -100,7 +104,8 @@ __global__ void __launch_bounds__(kThreads, MINB)
                     const double sg = s_ok ? P::kScale * gs[sj] : 0.0;
                     double ru = reaction[jb * 32 + lane].x, rv = reaction[jb * 32 + lane].y;
                     if (__all_sync(0xffffffffu, all_ok && s_ok)) {
-                        sym::react_tiles_full<P, T>(g, tx, ty, tg, sx, sy, sg, u, v, ru, rv);
+                        sym::react_tiles_full<P, T, kBuffered>(g, tx, ty, tg, sx, sy, sg, src,
+                                                               near, u, v, ru, rv);
                     } else {
 #pragma unroll
                         for (int t = 0; t < T; ++t)
@@ -123,7 +128,9 @@ __global__ void __launch_bounds__(kThreads, MINB)
                 const bool t_ok = ti < n;
                 const double tx = t_ok ? x[ti] : 0.0, ty = t_ok ? y[ti] : 0.0;
                 const double tg = t_ok ? P::kScale * gs[ti] : 0.0;
-                double u = 0.0, v = 0.0;
+                const double tx1[1] = {tx}, ty1[1] = {ty}, tg1[1] = {tg};
+                double u1[1] = {0.0}, v1[1] = {0.0};
+                double &u = u1[0], &v = v1[0];
                 for (int jb = diagonal ? ib : 0; jb < a; ++jb) {
                     const size_t sj = J * block_len + static_cast<size_t>(jb) * 32 + lane;
                     const int s_ok = sj < n ? 1 : 0;
@@ -134,7 +141,12 @@ __global__ void __launch_bounds__(kThreads, MINB)
                         continue;
                     }
                     double ru = reaction[jb * 32 + lane].x, rv = reaction[jb * 32 + lane].y;
-                    sym::react_tile<P>(g, tx, ty, tg, t_ok, sx, sy, sg, s_ok, u, v, ru, rv);
+                    if (__all_sync(0xffffffffu, t_ok && s_ok)) {
+                        sym::react_tiles_full<P, 1, kBuffered>(g, tx1, ty1, tg1, sx, sy, sg, src,
+                                                               P::near(g, tx, ty), u1, v1, ru, rv);
+                    } else {
+                        sym::react_tile<P>(g, tx, ty, tg, t_ok, sx, sy, sg, s_ok, u, v, ru, rv);
+                    }
                     reaction[jb * 32 + lane] = make_double2(ru, rv);
                 }
                 if (diagonal) {  // reactions from the sub-blocks before this one in the same block
@@ -328,7 +340,11 @@ enum SymKernel : int {
     SYM_PERIODIC_7 = 6,   // the periodic FP64 kernel built for 7 resident CTAs per SM
     SYM_PERIODIC_8 = 7,   // ... and for 8
     SYM_PERIODIC_T2 = 8,  // the periodic FP64 kernel with two targets per lane off the diagonal
-    SYM_KERNELS = 9
+    SYM_ZETA = 9,         // the periodic FP64 kernels with the rational pair term, the same forms
+    SYM_ZETA_7 = 10,
+    SYM_ZETA_8 = 11,
+    SYM_ZETA_T2 = 12,
+    SYM_KERNELS = 13
 };
 
 int kernel_of(const SymmetricPlan &p) {
@@ -340,7 +356,9 @@ int kernel_of(const SymmetricPlan &p) {
     if (fp32c)
         return SYM_PERIODIC32;
     if (p.targets == 2)
-        return SYM_PERIODIC_T2;
+        return p.zeta ? SYM_ZETA_T2 : SYM_PERIODIC_T2;
+    if (p.zeta)
+        return p.min_ctas == 8 ? SYM_ZETA_8 : (p.min_ctas == 7 ? SYM_ZETA_7 : SYM_ZETA);
     return p.min_ctas == 8 ? SYM_PERIODIC_8 : (p.min_ctas == 7 ? SYM_PERIODIC_7 : SYM_PERIODIC);
 }
 
@@ -368,7 +386,7 @@ int resident_ctas(int a, int kernel) {
             blocks = occupancy(symmetric32_kernel<f32::Periodic32, 1>, smem);
             break;
         case SYM_PLANE:
-            blocks = occupancy(symmetric_kernel<sym::PlaneSym, kPlaneTargets>, smem);
+            blocks = occupancy(symmetric_kernel<sym::PlaneSym, kPlaneTargets, 6>, smem);
             break;
         case SYM_PLANE_WIDE:
             blocks = occupancy(symmetric_kernel<sym::PlaneSym, kPlaneTargetsWide>, smem);
@@ -387,6 +405,18 @@ int resident_ctas(int a, int kernel) {
             break;
         case SYM_PERIODIC_T2:
             blocks = occupancy(symmetric_kernel<sym::PeriodicSym, 2>, smem);
+            break;
+        case SYM_ZETA:
+            blocks = occupancy(symmetric_kernel<sym::ZetaSym, 1>, smem);
+            break;
+        case SYM_ZETA_7:
+            blocks = occupancy(symmetric_kernel<sym::ZetaSym, 1, 7>, smem);
+            break;
+        case SYM_ZETA_8:
+            blocks = occupancy(symmetric_kernel<sym::ZetaSym, 1, 8>, smem);
+            break;
+        case SYM_ZETA_T2:
+            blocks = occupancy(symmetric_kernel<sym::ZetaSym, 2>, smem);
             break;
         default:
             blocks = occupancy(symmetric_kernel<sym::PeriodicSym, 1>, smem);
@@ -453,7 +483,8 @@ bool symmetric_tuning_store(int geometry, int precision, int log2_n, int mode, i
     return true;
 }
 
-SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, int geometry) {
+SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const GeometryConsts &g) {
+    const int geometry = g.geometry;
     SymmetricPlan p{};
     const bool plane = geometry == GEO_INFINITE;
     if (!plane && geometry != GEO_PERIODIC)
@@ -492,6 +523,7 @@ SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, int geometry
             p.items = static_cast<unsigned>(blocks * (blocks + 1) / 2);
             p.precision = precision;
             p.geometry = geometry;
+            p.zeta = g.zeta;
             p.targets = targets;
             const int fit = resident_ctas(a, kernel_of(p));
             const int want = symmetric_grid_lookup(geometry, precision, n);
@@ -524,7 +556,7 @@ cudaError_t launch_symmetric(const double *x, const double *y, const double *gs,
         return launch_pdl(symmetric32_kernel<f32::Periodic32, 1>, grid, block, smem, stream, x, y,
                           gs, n, p.a, items, p.items, counter, rows, stride, g, near);
     case SYM_PLANE:
-        return launch_pdl(symmetric_kernel<sym::PlaneSym, kPlaneTargets>, grid, block, smem,
+        return launch_pdl(symmetric_kernel<sym::PlaneSym, kPlaneTargets, 6>, grid, block, smem,
                           stream, x, y, gs, n, p.a, items, p.items, counter, rows, stride, g);
     case SYM_PLANE_WIDE:
         return launch_pdl(symmetric_kernel<sym::PlaneSym, kPlaneTargetsWide>, grid, block, smem,
@@ -543,6 +575,18 @@ cudaError_t launch_symmetric(const double *x, const double *y, const double *gs,
     case SYM_PERIODIC_8:
         return launch_pdl(symmetric_kernel<sym::PeriodicSym, 1, 8>, grid, block, smem, stream, x, y,
                           gs, n, p.a, items, p.items, counter, rows, stride, g);
+    case SYM_ZETA:
+        return launch_pdl(symmetric_kernel<sym::ZetaSym, 1>, grid, block, smem, stream, x, y, gs, n,
+                          p.a, items, p.items, counter, rows, stride, g);
+    case SYM_ZETA_7:
+        return launch_pdl(symmetric_kernel<sym::ZetaSym, 1, 7>, grid, block, smem, stream, x, y, gs,
+                          n, p.a, items, p.items, counter, rows, stride, g);
+    case SYM_ZETA_8:
+        return launch_pdl(symmetric_kernel<sym::ZetaSym, 1, 8>, grid, block, smem, stream, x, y, gs,
+                          n, p.a, items, p.items, counter, rows, stride, g);
+    case SYM_ZETA_T2:
+        return launch_pdl(symmetric_kernel<sym::ZetaSym, 2>, grid, block, smem, stream, x, y, gs, n,
+                          p.a, items, p.items, counter, rows, stride, g);
     case SYM_PERIODIC_T2:
         return launch_pdl(symmetric_kernel<sym::PeriodicSym, 2>, grid, block, smem, stream, x, y,
                           gs, n, p.a, items, p.items, counter, rows, stride, g);

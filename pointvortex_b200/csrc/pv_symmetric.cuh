@@ -33,6 +33,32 @@ struct PeriodicSym {
         ku = au * rcp_refined(bu);
         kv = av * rcp_refined(bv);
     }
+    static constexpr bool kNearForm = false;
+    __device__ __forceinline__ static bool near(const GeometryConsts &, double, double) {
+        return false;
+    }
+};
+
+// The box from six images up (ZetaPair). Tiles whose vortices are all in or near the box reduce a
+// difference by one subtraction (values_near): two FP64 instructions an axis with it, four without
+// (a population that has drifted out of the box: 8 % more of the pair's 50).
+struct ZetaSym {
+    static constexpr double kScale = 1.0;
+    static constexpr bool kNearForm = true;
+    __device__ __forceinline__ static void values(const GeometryConsts &g, double tx, double ty,
+                                                  double sx, double sy, double &ku, double &kv) {
+        ZetaPair::terms(g, ZetaPair::reduce(g, tx - sx, g.lx, g.inv_lx),
+                        ZetaPair::reduce(g, ty - sy, g.ly, g.inv_ly), ku, kv);
+    }
+    __device__ __forceinline__ static void values_near(const GeometryConsts &g, double tx,
+                                                       double ty, double sx, double sy,
+                                                       double &ku, double &kv) {
+        ZetaPair::terms(g, ZetaPair::reduce_near(g, tx - sx, g.lx),
+                        ZetaPair::reduce_near(g, ty - sy, g.ly), ku, kv);
+    }
+    __device__ __forceinline__ static bool near(const GeometryConsts &g, double x, double y) {
+        return ZetaPair::inside(g, x, y);
+    }
 };
 
 // The infinite plane (InfinitePair): K = (dy, dx) / (r^2 + eps^2), exactly odd in (dx, dy).
@@ -44,6 +70,10 @@ struct PlaneSym {
         const double inv = rcp_refined(fma(dx, dx, fma(dy, dy, g.eps2)));
         ku = dy * inv;
         kv = dx * inv;
+    }
+    static constexpr bool kNearForm = false;
+    __device__ __forceinline__ static bool near(const GeometryConsts &, double, double) {
+        return false;
     }
 };
 
@@ -87,14 +117,64 @@ __device__ __forceinline__ void react_tile(const GeometryConsts &g, double tx, d
         react_tile_t<P, false>(g, tx, ty, tg, t_ok, sx, sy, sg, s_ok, u, v, ru, rv);
 }
 
-// T targets per lane (T sub-blocks of targets) against one sub-block of 32 sources, every target
-// and source present. Each rotation step serves T pairs, so the shuffles (five doubles a step)
-// per pair fall by T: for a cheap pair term (the plane's) they would otherwise bound the tile.
-template <class P, int T>
-__device__ __forceinline__ void react_tiles_full(const GeometryConsts &g, const double (&tx)[T],
+// The sources of a tile in the warp's shared buffer, each twice, 32 entries apart, so that step k of
+// lane l reads entry l + k without a wrap.
+struct SourceBuffer {
+    double2 xy[64];
+    double g[64];
+    __device__ __forceinline__ void fill(double sx, double sy, double sg) {
+        const int lane = threadIdx.x & 31;
+        __syncwarp();  // the previous tile's reads are done
+        xy[lane] = xy[lane + 32] = make_double2(sx, sy);
+        g[lane] = g[lane + 32] = sg;
+        __syncwarp();
+    }
+};
+
+// T targets per lane (T sub-blocks of targets) against the 32 sources of the buffer, every target
+// and source present. Only the reactions rotate (two double shuffles a step, shared by the T
+// pairs); reading the sources instead of rotating them too (five) is 6 % faster with the box's
+// terms (N = 16384, T = 1: 500 against 532 us; T = 2: 472 against 493 us). U steps are unrolled:
+// two with one target per lane, four with two.
+template <class P, int T, bool NEAR, int U = (T == 2 ? 4 : 2)>
+__device__ __forceinline__ void react_tiles_steps(const GeometryConsts &g, const double (&tx)[T],
                                                  const double (&ty)[T], const double (&tg)[T],
-                                                 double sx, double sy, double sg, double (&u)[T],
+                                                 const SourceBuffer &b, double (&u)[T],
                                                  double (&v)[T], double &ru, double &rv) {
+    const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
+    const double2 *xy = b.xy + lane;
+    const double *sgs = b.g + lane;
+#pragma unroll U
+    for (int k = 0; k < 32; ++k) {
+        const double2 s = xy[k];
+        const double sg = sgs[k];
+#pragma unroll
+        for (int t = 0; t < T; ++t) {
+            double ku, kv;
+            if constexpr (NEAR)
+                P::values_near(g, tx[t], ty[t], s.x, s.y, ku, kv);
+            else
+                P::values(g, tx[t], ty[t], s.x, s.y, ku, kv);
+            u[t] = fma(-sg, ku, u[t]);    // target: -c_s K
+            v[t] = fma(sg, kv, v[t]);
+            ru = fma(tg[t], ku, ru);      // source: the exchanged pair, +c_t K
+            rv = fma(-tg[t], kv, rv);
+        }
+        ru = rotate(ru, next);
+        rv = rotate(rv, next);
+    }
+}
+
+// The same with the sources rotating through the lanes beside their reactions. With eight targets
+// per lane (the plane's wide form) the shuffles of a step are shared by eight pairs, and reading
+// the sources instead is slower: launches of 1204 against 1175 us at N = 50 001, 1919 against
+// 1892 us at 65 536.
+template <class P, int T>
+__device__ __forceinline__ void react_tiles_rotating(const GeometryConsts &g,
+                                                     const double (&tx)[T], const double (&ty)[T],
+                                                     const double (&tg)[T], double sx, double sy,
+                                                     double sg, double (&u)[T], double (&v)[T],
+                                                     double &ru, double &rv) {
     const int next = (threadIdx.x + 1) & 31;
 #pragma unroll 2
     for (int k = 0; k < 32; ++k) {
@@ -113,6 +193,27 @@ __device__ __forceinline__ void react_tiles_full(const GeometryConsts &g, const 
         ru = rotate(ru, next);
         rv = rotate(rv, next);
     }
+}
+
+// One whole tile set of T targets per lane. near: this lane's targets satisfy P::near.
+template <class P, int T, bool BUFFERED>
+__device__ __forceinline__ void react_tiles_full(const GeometryConsts &g, const double (&tx)[T],
+                                                 const double (&ty)[T], const double (&tg)[T],
+                                                 double sx, double sy, double sg, SourceBuffer &b,
+                                                 bool near, double (&u)[T], double (&v)[T],
+                                                 double &ru, double &rv) {
+    if constexpr (!BUFFERED) {
+        react_tiles_rotating<P, T>(g, tx, ty, tg, sx, sy, sg, u, v, ru, rv);
+        return;
+    }
+    b.fill(sx, sy, sg);
+    if constexpr (P::kNearForm) {
+        if (__all_sync(0xffffffffu, near && P::near(g, sx, sy))) {
+            react_tiles_steps<P, T, true>(g, tx, ty, tg, b, u, v, ru, rv);
+            return;
+        }
+    }
+    react_tiles_steps<P, T, false>(g, tx, ty, tg, b, u, v, ru, rv);
 }
 
 // Target side only. same_block: the sources are the targets' own lanes, so the self pair (k = 0)

@@ -217,8 +217,9 @@ bool tuning_store(int geometry, int precision, int log2_n, int per_thread) {
     return true;
 }
 
-EvalPlan plan_evaluation(int geometry, size_t n_targets, size_t n_sources, int sm_count,
+EvalPlan plan_evaluation(const GeometryConsts &g, size_t n_targets, size_t n_sources, int sm_count,
                          int per_thread_override, int precision) {
+    const int geometry = g.geometry;
     EvalPlan p{};
     p.block = 128;
     if (per_thread_override == 0)
@@ -232,7 +233,8 @@ EvalPlan plan_evaluation(int geometry, size_t n_targets, size_t n_sources, int s
         if (precision == 1)
             return resident_fp32c(geometry, t);
         return geometry == GEO_INFINITE   ? resident_for<InfinitePair>(t)
-               : geometry == GEO_PERIODIC ? resident_for<PeriodicPair>(t)
+               : geometry == GEO_PERIODIC ? (g.zeta ? resident_for<ZetaPair>(t)
+                                                    : resident_for<PeriodicPair>(t))
                                           : resident_for<DiskPair>(t);
     };
     const auto blocks_of = [&](int t) {
@@ -285,7 +287,8 @@ cudaError_t launch_velocity(const EvalArgs &a, const EvalPlan &p, cudaStream_t s
     case GEO_INFINITE:
         return launch_pair<InfinitePair>(a, p, stream);
     case GEO_PERIODIC:
-        return launch_pair<PeriodicPair>(a, p, stream);
+        return a.g.zeta ? launch_pair<ZetaPair>(a, p, stream)
+                        : launch_pair<PeriodicPair>(a, p, stream);
     case GEO_DISK:
         return launch_pair<DiskPair>(a, p, stream);
     default:
