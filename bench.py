@@ -487,7 +487,7 @@ def run_kernel_case(spec: str, evals: int, precision: str = "fp64", ordered: boo
     else:
         x, y, g = ics.disk(n, 3, 1.0)
         k = pv.DiskKernel(1.0, precision=prec)
-        flops, flops_sym = 33, None
+        flops, flops_sym = 33, 47
     k.uploadDeviceState(pv.VortexSystem(x, y, g))
     symmetric = k.statePlan()["symmetric"] and not ordered
     run = (lambda: k.evaluate(x, y, g)) if ordered else k.evaluateDeviceState

@@ -247,6 +247,7 @@ __device__ __forceinline__ void run_item(const GeometryConsts &g, const double *
 // targets I*128 + 32w + lane and meets the four 32-source sub-tiles of block J in turn. Targets'
 // sums go to row J, the sources' reactions (summed over the four warps in fixed order) to row I.
 // A diagonal item (I == J) is evaluated one-sided. red_u / red_v: 4 x 128 doubles of shared memory.
+template <class P>
 __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, const double *px,
                                                    const double *py, const double *sgs, size_t n,
                                                    unsigned I, unsigned J, double *pu, double *pv,
@@ -255,20 +256,24 @@ __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, cons
     const bool diagonal = I == J;
     const size_t ti = static_cast<size_t>(I) * kBlock + static_cast<size_t>(w) * 32 + lane;
     const bool t_ok = ti < n;
-    const double tx = t_ok ? px[ti] : 0.0, ty = t_ok ? py[ti] : 0.0;
-    const double tg2 = t_ok ? 2.0 * sgs[ti] : 0.0;  // doubled: the terms carry half sines
+    const auto vortex = [&](size_t i) {
+        return i < n ? sym::Vortex{px[i], py[i], P::kScale * sgs[i]} : sym::Vortex{0.0, 0.0, 0.0};
+    };
+    const sym::Vortex t = vortex(ti);
     double u = 0.0, v = 0.0;
     for (int qq = 0; qq < 4; ++qq) {
         const int q = (w + qq) & 3;
         const size_t sj = static_cast<size_t>(J) * kBlock + static_cast<size_t>(q) * 32 + lane;
         const int s_ok = sj < n ? 1 : 0;
-        const double sx = s_ok ? px[sj] : 0.0, sy = s_ok ? py[sj] : 0.0;
-        const double sg2 = s_ok ? 2.0 * sgs[sj] : 0.0;
+        const sym::Vortex s = vortex(sj);
         if (diagonal) {
-            sym::one_sided_tile(g, tx, ty, t_ok, sx, sy, sg2, s_ok, q == w, u, v);
+            sym::one_sided_tile<P>(g, t, t_ok, s, s_ok, q == w, u, v);
         } else {
             double ru = 0.0, rv = 0.0;
-            sym::react_tile(g, tx, ty, tg2, t_ok, sx, sy, sg2, s_ok, u, v, ru, rv);
+            if (__all_sync(0xffffffffu, t_ok && s_ok))
+                sym::react_tile_t<P, true>(g, t, t_ok, s, s_ok, u, v, ru, rv);
+            else
+                sym::react_tile_t<P, false>(g, t, t_ok, s, s_ok, u, v, ru, rv);
             red_u[w * kBlock + q * 32 + lane] = ru;
             red_v[w * kBlock + q * 32 + lane] = rv;
         }
@@ -584,7 +589,7 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
                 run_symmetric_item32(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu, pv, d.pad_n,
                                      &s_x[0][0], &s_y[0][0], s_f, s_gf);
             else
-                run_symmetric_item(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu, pv, d.pad_n,
+                run_symmetric_item<sym::PeriodicSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu, pv, d.pad_n,
                                    &s_x[0][0], &s_y[0][0]);
             __syncthreads();
             continue;

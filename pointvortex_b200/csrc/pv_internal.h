@@ -71,7 +71,7 @@ cudaError_t launch_velocity_fp32c(const EvalArgs &a, const EvalPlan &p, cudaStre
 // Resident CTAs per SM of the FP32-compensated ordered kernel (the planner's wave arithmetic).
 int resident_fp32c(int geometry, int per_thread);
 
-// The periodic box and the infinite plane (FP64, FP32C) evaluated once per unordered pair
+// The periodic box and the infinite plane (FP64, FP32C) and the FP64 disk once per unordered pair
 // (pv_symmetric.cu) for a whole population (targets = sources). Partial rows: `blocks` rows of
 // `stride` (u, v) pairs, row r of vortex i at rows[r * stride + i].
 struct SymmetricPlan {
@@ -80,7 +80,7 @@ struct SymmetricPlan {
     unsigned items = 0;  // block pairs (I <= J)
     int grid = 0;        // persistent CTAs
     int precision = 0;   // PV_PRECISION_FP64 or PV_PRECISION_FP32C
-    int geometry = 0;    // GEO_PERIODIC or GEO_INFINITE
+    int geometry = 0;
     int zeta = 0;        // periodic FP64: the rational pair term (ZetaPair)
     int targets = 1;     // targets per lane off the diagonal (the plane: 4 or 8)
     int min_ctas = 0;    // periodic FP64: the kernel built for 7 or 8 CTAs per SM (0: default)
@@ -91,6 +91,12 @@ constexpr size_t kSymmetricMinN = 2048;       // periodic box below: the ordered
 constexpr size_t kSymmetricPlaneMinN = 16384;   // infinite plane below: the ordered kernel
 constexpr size_t kSymmetricPlane32MinN = 16384; // the same for the FP32-compensated plane
 constexpr size_t kSymmetricPlaneWideN = 32768;  // the plane from here: 8 targets per lane
+// FP64 disk below: the ordered kernel (18 us at 2048; the once-per-pair tiles 19, 36 against 43 at
+// 4096, where 128 blocks of 32 first give every SM work)
+constexpr size_t kSymmetricDiskMinN = 4096;
+// the disk from here 4 targets per lane, from half of it 2 (16 384: 314 against 326 us with 2;
+// 8192: 100 with 2 against 102 with 1; more per lane leaves too few items)
+constexpr size_t kSymmetricDiskWideN = 16384;
 constexpr size_t kSymmetricPartialBytes = static_cast<size_t>(256) << 20;  // a grows past this
 constexpr size_t kSymmetricPartialBytesMax = static_cast<size_t>(4) << 30;  // beyond: ordered kernel
 SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const GeometryConsts &g);

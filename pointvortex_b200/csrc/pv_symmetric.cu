@@ -81,44 +81,44 @@ __global__ void __launch_bounds__(kThreads, MINB)
         const bool diagonal = I == J;
         for (int jb = 0; jb < a; ++jb)
             reaction[jb * 32 + lane] = make_double2(0.0, 0.0);
+        const auto vortex = [&](size_t i) {
+            return i < n ? sym::Vortex{x[i], y[i], P::kScale * gs[i]} : sym::Vortex{0.0, 0.0, 0.0};
+        };
         if (T > 1 && !diagonal) {
             for (int ib = 0; ib < a; ib += T) {
-                double tx[T], ty[T], tg[T], u[T], v[T];
+                sym::Vortex t[T];
+                double u[T], v[T];
                 bool t_ok[T], all_ok = true, near = true;
 #pragma unroll
-                for (int t = 0; t < T; ++t) {
-                    const size_t ti = I * block_len + static_cast<size_t>(ib + t) * 32 + lane;
-                    t_ok[t] = ti < n;
-                    all_ok = all_ok && t_ok[t];
-                    tx[t] = t_ok[t] ? x[ti] : 0.0;
-                    ty[t] = t_ok[t] ? y[ti] : 0.0;
-                    tg[t] = t_ok[t] ? P::kScale * gs[ti] : 0.0;
-                    near = near && P::near(g, tx[t], ty[t]);
-                    u[t] = 0.0;
-                    v[t] = 0.0;
+                for (int q = 0; q < T; ++q) {
+                    const size_t ti = I * block_len + static_cast<size_t>(ib + q) * 32 + lane;
+                    t_ok[q] = ti < n;
+                    all_ok = all_ok && t_ok[q];
+                    t[q] = vortex(ti);
+                    near = near && P::near(g, t[q].x, t[q].y);
+                    u[q] = 0.0;
+                    v[q] = 0.0;
                 }
                 for (int jb = 0; jb < a; ++jb) {
                     const size_t sj = J * block_len + static_cast<size_t>(jb) * 32 + lane;
                     const int s_ok = sj < n ? 1 : 0;
-                    const double sx = s_ok ? x[sj] : 0.0, sy = s_ok ? y[sj] : 0.0;
-                    const double sg = s_ok ? P::kScale * gs[sj] : 0.0;
+                    const sym::Vortex s = vortex(sj);
                     double ru = reaction[jb * 32 + lane].x, rv = reaction[jb * 32 + lane].y;
                     if (__all_sync(0xffffffffu, all_ok && s_ok)) {
-                        sym::react_tiles_full<P, T, kBuffered>(g, tx, ty, tg, sx, sy, sg, src,
-                                                               near, u, v, ru, rv);
+                        sym::react_tiles_full<P, T, kBuffered>(g, t, s, src, near, u, v, ru, rv);
                     } else {
 #pragma unroll
-                        for (int t = 0; t < T; ++t)
-                            sym::react_tile<P>(g, tx[t], ty[t], tg[t], t_ok[t], sx, sy, sg, s_ok,
-                                               u[t], v[t], ru, rv);
+                        for (int q = 0; q < T; ++q)
+                            sym::react_tile_t<P, false>(g, t[q], t_ok[q], s, s_ok, u[q], v[q], ru,
+                                                        rv);
                     }
                     reaction[jb * 32 + lane] = make_double2(ru, rv);
                 }
 #pragma unroll
-                for (int t = 0; t < T; ++t) {
-                    const size_t ti = I * block_len + static_cast<size_t>(ib + t) * 32 + lane;
-                    if (t_ok[t]) {
-                        pr[J * stride + ti] = make_double2(u[t], v[t]);
+                for (int q = 0; q < T; ++q) {
+                    const size_t ti = I * block_len + static_cast<size_t>(ib + q) * 32 + lane;
+                    if (t_ok[q]) {
+                        pr[J * stride + ti] = make_double2(u[q], v[q]);
                     }
                 }
             }
@@ -126,36 +126,31 @@ __global__ void __launch_bounds__(kThreads, MINB)
             for (int ib = 0; ib < a; ++ib) {
                 const size_t ti = I * block_len + static_cast<size_t>(ib) * 32 + lane;
                 const bool t_ok = ti < n;
-                const double tx = t_ok ? x[ti] : 0.0, ty = t_ok ? y[ti] : 0.0;
-                const double tg = t_ok ? P::kScale * gs[ti] : 0.0;
-                const double tx1[1] = {tx}, ty1[1] = {ty}, tg1[1] = {tg};
-                double u1[1] = {0.0}, v1[1] = {0.0};
-                double &u = u1[0], &v = v1[0];
+                const sym::Vortex t[1] = {vortex(ti)};
+                double u[1] = {0.0}, v[1] = {0.0};
                 for (int jb = diagonal ? ib : 0; jb < a; ++jb) {
                     const size_t sj = J * block_len + static_cast<size_t>(jb) * 32 + lane;
                     const int s_ok = sj < n ? 1 : 0;
-                    const double sx = s_ok ? x[sj] : 0.0, sy = s_ok ? y[sj] : 0.0;
-                    const double sg = s_ok ? P::kScale * gs[sj] : 0.0;
+                    const sym::Vortex s = vortex(sj);
                     if (diagonal && jb == ib) {
-                        sym::one_sided_tile<P>(g, tx, ty, t_ok, sx, sy, sg, s_ok, true, u, v);
+                        sym::one_sided_tile<P>(g, t[0], t_ok, s, s_ok, true, u[0], v[0]);
                         continue;
                     }
                     double ru = reaction[jb * 32 + lane].x, rv = reaction[jb * 32 + lane].y;
-                    if (__all_sync(0xffffffffu, t_ok && s_ok)) {
-                        sym::react_tiles_full<P, 1, kBuffered>(g, tx1, ty1, tg1, sx, sy, sg, src,
-                                                               P::near(g, tx, ty), u1, v1, ru, rv);
-                    } else {
-                        sym::react_tile<P>(g, tx, ty, tg, t_ok, sx, sy, sg, s_ok, u, v, ru, rv);
-                    }
+                    if (__all_sync(0xffffffffu, t_ok && s_ok))
+                        sym::react_tiles_full<P, 1, kBuffered>(
+                            g, t, s, src, P::near(g, t[0].x, t[0].y), u, v, ru, rv);
+                    else
+                        sym::react_tile_t<P, false>(g, t[0], t_ok, s, s_ok, u[0], v[0], ru, rv);
                     reaction[jb * 32 + lane] = make_double2(ru, rv);
                 }
                 if (diagonal) {  // reactions from the sub-blocks before this one in the same block
                     const double2 r = reaction[ib * 32 + lane];
-                    u += r.x;
-                    v += r.y;
+                    u[0] += r.x;
+                    v[0] += r.y;
                 }
                 if (t_ok) {
-                    pr[J * stride + ti] = make_double2(u, v);
+                    pr[J * stride + ti] = make_double2(u[0], v[0]);
                 }
             }
         }
@@ -344,7 +339,10 @@ enum SymKernel : int {
     SYM_ZETA_7 = 10,
     SYM_ZETA_8 = 11,
     SYM_ZETA_T2 = 12,
-    SYM_KERNELS = 13
+    SYM_DISK = 13,        // the disk with one, two and four targets per lane
+    SYM_DISK_T2 = 14,
+    SYM_DISK_T4 = 15,
+    SYM_KERNELS = 16
 };
 
 int kernel_of(const SymmetricPlan &p) {
@@ -353,6 +351,8 @@ int kernel_of(const SymmetricPlan &p) {
         const bool wide = p.targets == kPlaneTargetsWide;
         return fp32c ? (wide ? SYM_PLANE32_WIDE : SYM_PLANE32) : (wide ? SYM_PLANE_WIDE : SYM_PLANE);
     }
+    if (p.geometry == GEO_DISK)
+        return p.targets == 4 ? SYM_DISK_T4 : (p.targets == 2 ? SYM_DISK_T2 : SYM_DISK);
     if (fp32c)
         return SYM_PERIODIC32;
     if (p.targets == 2)
@@ -406,6 +406,15 @@ int resident_ctas(int a, int kernel) {
         case SYM_PERIODIC_T2:
             blocks = occupancy(symmetric_kernel<sym::PeriodicSym, 2>, smem);
             break;
+        case SYM_DISK:
+            blocks = occupancy(symmetric_kernel<sym::DiskSym, 1>, smem);
+            break;
+        case SYM_DISK_T2:
+            blocks = occupancy(symmetric_kernel<sym::DiskSym, 2>, smem);
+            break;
+        case SYM_DISK_T4:
+            blocks = occupancy(symmetric_kernel<sym::DiskSym, 4>, smem);
+            break;
         case SYM_ZETA:
             blocks = occupancy(symmetric_kernel<sym::ZetaSym, 1>, smem);
             break;
@@ -416,7 +425,7 @@ int resident_ctas(int a, int kernel) {
             blocks = occupancy(symmetric_kernel<sym::ZetaSym, 1, 8>, smem);
             break;
         case SYM_ZETA_T2:
-            blocks = occupancy(symmetric_kernel<sym::ZetaSym, 2>, smem);
+            blocks = occupancy(symmetric_kernel<sym::ZetaSym, 2, 5>, smem);
             break;
         default:
             blocks = occupancy(symmetric_kernel<sym::PeriodicSym, 1>, smem);
@@ -487,7 +496,8 @@ SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const Geomet
     const int geometry = g.geometry;
     SymmetricPlan p{};
     const bool plane = geometry == GEO_INFINITE;
-    if (!plane && geometry != GEO_PERIODIC)
+    const bool disk = geometry == GEO_DISK;
+    if (disk && precision == PV_PRECISION_FP32C)
         return p;
     // the measured table overrides the built-in choice of form, occupancy and targets per lane
     const int tuned = symmetric_tuning_lookup(geometry, precision, n);
@@ -496,7 +506,7 @@ SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const Geomet
         return p;
     const size_t min_n = plane ? (precision == PV_PRECISION_FP32C ? kSymmetricPlane32MinN
                                                                   : kSymmetricPlaneMinN)
-                               : kSymmetricMinN;
+                               : (disk ? kSymmetricDiskMinN : kSymmetricMinN);
     if (mode != 2 && n < min_n)
         return p;
     if (n < 64)
@@ -508,6 +518,7 @@ SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const Geomet
     const int targets =
         plane ? (tuned_targets ? tuned_targets
                                : (n >= kSymmetricPlaneWideN ? kPlaneTargetsWide : kPlaneTargets))
+        : disk ? (n >= kSymmetricDiskWideN ? 4 : (n >= kSymmetricDiskWideN / 2 ? 2 : 1))
               : (precision == PV_PRECISION_FP64 && tuned_targets == 2 ? 2 : 1);
     p.min_ctas = tuned_ctas;
     const size_t np = (n + 255) & ~static_cast<size_t>(255);
@@ -575,6 +586,15 @@ cudaError_t launch_symmetric(const double *x, const double *y, const double *gs,
     case SYM_PERIODIC_8:
         return launch_pdl(symmetric_kernel<sym::PeriodicSym, 1, 8>, grid, block, smem, stream, x, y,
                           gs, n, p.a, items, p.items, counter, rows, stride, g);
+    case SYM_DISK:
+        return launch_pdl(symmetric_kernel<sym::DiskSym, 1>, grid, block, smem, stream, x, y, gs, n,
+                          p.a, items, p.items, counter, rows, stride, g);
+    case SYM_DISK_T2:
+        return launch_pdl(symmetric_kernel<sym::DiskSym, 2>, grid, block, smem, stream, x, y, gs, n,
+                          p.a, items, p.items, counter, rows, stride, g);
+    case SYM_DISK_T4:
+        return launch_pdl(symmetric_kernel<sym::DiskSym, 4>, grid, block, smem, stream, x, y, gs, n,
+                          p.a, items, p.items, counter, rows, stride, g);
     case SYM_ZETA:
         return launch_pdl(symmetric_kernel<sym::ZetaSym, 1>, grid, block, smem, stream, x, y, gs, n,
                           p.a, items, p.items, counter, rows, stride, g);
@@ -585,7 +605,7 @@ cudaError_t launch_symmetric(const double *x, const double *y, const double *gs,
         return launch_pdl(symmetric_kernel<sym::ZetaSym, 1, 8>, grid, block, smem, stream, x, y, gs,
                           n, p.a, items, p.items, counter, rows, stride, g);
     case SYM_ZETA_T2:
-        return launch_pdl(symmetric_kernel<sym::ZetaSym, 2>, grid, block, smem, stream, x, y, gs, n,
+        return launch_pdl(symmetric_kernel<sym::ZetaSym, 2, 5>, grid, block, smem, stream, x, y, gs, n,
                           p.a, items, p.items, counter, rows, stride, g);
     case SYM_PERIODIC_T2:
         return launch_pdl(symmetric_kernel<sym::PeriodicSym, 2>, grid, block, smem, stream, x, y,

@@ -1,13 +1,13 @@
-// pv_symmetric.cuh — warp tiles evaluated once per unordered pair (periodic box, infinite plane),
+// pv_symmetric.cuh — warp tiles evaluated once per unordered pair (box, plane, disk),
 // shared by the single-simulation kernels (pv_symmetric.cu) and the batched ensembles
 // (pv_batch.cu).
 //
-// A tile is 32 targets (one per lane) against 32 sources. The sources, with the reactions they
-// accumulate, rotate one lane per step by shuffles; after 32 steps every (target, source) pair has
-// been met once and every source is back in its home lane. The pair terms are exactly odd under
-// exchanging target and source, so one evaluation gives the target's term and, with the other
-// circulation and the opposite sign, the source's. Callers pass the scaled circulations times
-// the policy's kScale (the periodic terms carry half sines: 2 * Gamma * 0.5/L).
+// A tile is 32 targets (one per lane) against 32 sources. The reactions that the sources
+// accumulate rotate one lane per step by shuffles; after 32 steps every (target, source) pair has
+// been met once and every reaction is back in its home lane. What a pair's two terms have in
+// common is evaluated once: in the box and the plane everything but the circulation and the sign,
+// in the disk the two reciprocals. Callers pass the scaled circulations times the policy's kScale
+// (PeriodicSym's terms carry half sines: 2 * Gamma * 0.5/L).
 #pragma once
 
 #include "pv_geometry.cuh"
@@ -20,10 +20,51 @@ __device__ __forceinline__ double rotate(double v, int from) {
     return __shfl_sync(0xffffffffu, v, from);
 }
 
-// Pair kernels K of the geometries evaluated this way: the target's velocity changes by
-// u -= c_s K_u, v += c_s K_v and the source's by u += c_t K_u, v -= c_t K_v, where c is the
-// stored scaled circulation times kScale.
-struct PeriodicSym {
+// One vortex of a tile: position and the scaled circulation times the policy's kScale.
+struct Vortex {
+    double x, y, g;
+};
+
+// What the geometries evaluated this way provide:
+//   react<NEAR>(g, t, s, u, v, ru, rv): a pair's terms, the target's into (u, v) and the source's
+//     into (ru, rv). NEAR: all vortices of the tile satisfy near() (kNearForm policies only);
+//   one(g, t, s, u, v): the target's alone; self(g, t, u, v): what a vortex does to itself.
+//
+// The box and the plane have antisymmetric kernels K: the target's velocity changes by u -= c_s K_u,
+// v += c_s K_v and the source's by u += c_t K_u, v -= c_t K_v.
+template <class K> struct Antisymmetric {
+    static constexpr bool kNearForm = false;
+    static constexpr double kScale = 1.0;
+    __device__ __forceinline__ static bool near(const GeometryConsts &, double, double) {
+        return false;
+    }
+    template <bool NEAR>
+    __device__ __forceinline__ static void react(const GeometryConsts &g, const Vortex &t,
+                                                 const Vortex &s, double &u, double &v, double &ru,
+                                                 double &rv) {
+        double ku, kv;
+        if constexpr (NEAR)
+            K::values_near(g, t.x, t.y, s.x, s.y, ku, kv);
+        else
+            K::values(g, t.x, t.y, s.x, s.y, ku, kv);
+        u = fma(-s.g, ku, u);
+        v = fma(s.g, kv, v);
+        ru = fma(t.g, ku, ru);
+        rv = fma(-t.g, kv, rv);
+    }
+    __device__ __forceinline__ static void one(const GeometryConsts &g, const Vortex &t,
+                                               const Vortex &s, double &u, double &v) {
+        double ku, kv;
+        K::values(g, t.x, t.y, s.x, s.y, ku, kv);
+        u = fma(-s.g, ku, u);
+        v = fma(s.g, kv, v);
+    }
+    // the reference skips the self pair (and in the periodic box it contributes exactly 0)
+    __device__ __forceinline__ static void self(const GeometryConsts &, const Vortex &, double &,
+                                                double &) {}
+};
+
+struct PeriodicSym : Antisymmetric<PeriodicSym> {
     // the terms carry half sines (PeriodicPair::terms<true>): circulations are doubled
     static constexpr double kScale = 2.0;
     __device__ __forceinline__ static void values(const GeometryConsts &g, double tx, double ty,
@@ -33,17 +74,12 @@ struct PeriodicSym {
         ku = au * rcp_refined(bu);
         kv = av * rcp_refined(bv);
     }
-    static constexpr bool kNearForm = false;
-    __device__ __forceinline__ static bool near(const GeometryConsts &, double, double) {
-        return false;
-    }
 };
 
 // The box from six images up (ZetaPair). Tiles whose vortices are all in or near the box reduce a
 // difference by one subtraction (values_near): two FP64 instructions an axis with it, four without
 // (a population that has drifted out of the box: 8 % more of the pair's 50).
-struct ZetaSym {
-    static constexpr double kScale = 1.0;
+struct ZetaSym : Antisymmetric<ZetaSym> {
     static constexpr bool kNearForm = true;
     __device__ __forceinline__ static void values(const GeometryConsts &g, double tx, double ty,
                                                   double sx, double sy, double &ku, double &kv) {
@@ -62,8 +98,7 @@ struct ZetaSym {
 };
 
 // The infinite plane (InfinitePair): K = (dy, dx) / (r^2 + eps^2), exactly odd in (dx, dy).
-struct PlaneSym {
-    static constexpr double kScale = 1.0;
+struct PlaneSym : Antisymmetric<PlaneSym> {
     __device__ __forceinline__ static void values(const GeometryConsts &g, double tx, double ty,
                                                   double sx, double sy, double &ku, double &kv) {
         const double dx = tx - sx, dy = ty - sy;
@@ -71,34 +106,92 @@ struct PlaneSym {
         ku = dy * inv;
         kv = dx * inv;
     }
+};
+
+// The disk (DiskPair). The direct term is the plane's. For the wall images, with A = R^2 - t.s and
+// B = t x s (t_y s_x - t_x s_y), the target gets c_s (B s_x - A s_y, A s_x + B s_y) / (A^2 + B^2):
+// exchanging the vortices keeps A and negates B, so one reciprocal serves both sides. Beside the
+// circulations stand the moments c s and c t. 34 FP64 instructions an unordered pair (two of them
+// the source's moments, shared by the lane's targets) against 58 for its two ordered pairs;
+// measured per launch, ordered against this: N = 4096 43 -> 36 us, 8192 135 -> 100 us, 12 000
+// 294 -> 185 us, 16 384 504 -> 314 us, 40 000 2756 -> 1772 us. The FP64 pipe bounds it: 34
+// instructions of two or (18, all operands distinct registers) three cycles.
+struct DiskSym {
     static constexpr bool kNearForm = false;
+    static constexpr double kScale = 1.0;
     __device__ __forceinline__ static bool near(const GeometryConsts &, double, double) {
         return false;
     }
+    // (A, B) / (A^2 + B^2)
+    __device__ __forceinline__ static void image(const GeometryConsts &g, const Vortex &t,
+                                                 const Vortex &s, double &a, double &b) {
+        const double A = fma(-t.y, s.y, fma(-t.x, s.x, g.radius2));
+        const double B = fma(t.y, s.x, -t.x * s.y);
+        const double inv = rcp_refined(fma(A, A, B * B));
+        a = A * inv;
+        b = B * inv;
+    }
+    template <bool NEAR>
+    __device__ __forceinline__ static void react(const GeometryConsts &g, const Vortex &t,
+                                                 const Vortex &s, double &u, double &v, double &ru,
+                                                 double &rv) {
+        const double dx = t.x - s.x, dy = t.y - s.y;
+        const double inv = rcp_refined(fma(dx, dx, dy * dy));
+        const double ku = dy * inv, kv = dx * inv;
+        double a, b;
+        image(g, t, s, a, b);
+        const double smx = s.g * s.x, smy = s.g * s.y, tmx = t.g * t.x, tmy = t.g * t.y;
+        u = fma(-s.g, ku, u);
+        ru = fma(t.g, ku, ru);
+        v = fma(s.g, kv, v);
+        rv = fma(-t.g, kv, rv);
+        u = fma(b, smx, u);
+        v = fma(b, smy, v);
+        ru = fma(-b, tmx, ru);
+        rv = fma(-b, tmy, rv);
+        u = fma(-a, smy, u);
+        v = fma(a, smx, v);
+        ru = fma(-a, tmy, ru);
+        rv = fma(a, tmx, rv);
+    }
+    __device__ __forceinline__ static void one(const GeometryConsts &g, const Vortex &t,
+                                               const Vortex &s, double &u, double &v) {
+        const double dx = t.x - s.x, dy = t.y - s.y;
+        const double c = s.g * rcp_refined(fma(dx, dx, dy * dy));
+        u = fma(-c, dy, u);
+        v = fma(c, dx, v);
+        self_image(g, t, s, u, v);
+    }
+    __device__ __forceinline__ static void self_image(const GeometryConsts &g, const Vortex &t,
+                                                      const Vortex &s, double &u, double &v) {
+        double a, b;
+        image(g, t, s, a, b);
+        const double smx = s.g * s.x, smy = s.g * s.y;
+        u = fma(b, smx, fma(-a, smy, u));
+        v = fma(a, smx, fma(b, smy, v));
+    }
+    // a vortex meets its own image
+    __device__ __forceinline__ static void self(const GeometryConsts &g, const Vortex &t, double &u,
+                                                double &v) {
+        self_image(g, t, t, u, v);
+    }
 };
 
-// Targets (tx, ty, tg) against the sources held in the lanes (sx, sy, sg and their reactions
-// ru, rv); adds the targets' sums to u, v and the sources' to ru, rv. Sources end at home.
-// FULL: all 32 targets and sources exist (every tile but the last block's), no predicates.
+// Target t against the sources held in the lanes (s and their reactions ru, rv); adds the targets'
+// sums to u, v and the sources' to ru, rv. Sources end at home. FULL: all 32 targets and sources
+// exist, no predicates.
 template <class P, bool FULL>
-__device__ __forceinline__ void react_tile_t(const GeometryConsts &g, double tx, double ty,
-                                             double tg, bool t_ok, double sx, double sy,
-                                             double sg, int s_ok, double &u, double &v,
-                                             double &ru, double &rv) {
+__device__ __forceinline__ void react_tile_t(const GeometryConsts &g, const Vortex &t, bool t_ok,
+                                             Vortex s, int s_ok, double &u, double &v, double &ru,
+                                             double &rv) {
     const int next = (threadIdx.x + 1) & 31;
 #pragma unroll 2
     for (int k = 0; k < 32; ++k) {
-        if (FULL || (t_ok && s_ok)) {
-            double ku, kv;
-            P::values(g, tx, ty, sx, sy, ku, kv);
-            u = fma(-sg, ku, u);   // target: -c_s K
-            v = fma(sg, kv, v);
-            ru = fma(tg, ku, ru);  // source: the exchanged pair, +c_t K
-            rv = fma(-tg, kv, rv);
-        }
-        sx = rotate(sx, next);
-        sy = rotate(sy, next);
-        sg = rotate(sg, next);
+        if (FULL || (t_ok && s_ok))
+            P::template react<false>(g, t, s, u, v, ru, rv);
+        s.x = rotate(s.x, next);
+        s.y = rotate(s.y, next);
+        s.g = rotate(s.g, next);
         ru = rotate(ru, next);
         rv = rotate(rv, next);
         if (!FULL)
@@ -106,27 +199,16 @@ __device__ __forceinline__ void react_tile_t(const GeometryConsts &g, double tx,
     }
 }
 
-template <class P = PeriodicSym>
-__device__ __forceinline__ void react_tile(const GeometryConsts &g, double tx, double ty,
-                                           double tg, bool t_ok, double sx, double sy, double sg,
-                                           int s_ok, double &u, double &v, double &ru,
-                                           double &rv) {
-    if (__all_sync(0xffffffffu, t_ok && s_ok))
-        react_tile_t<P, true>(g, tx, ty, tg, t_ok, sx, sy, sg, s_ok, u, v, ru, rv);
-    else
-        react_tile_t<P, false>(g, tx, ty, tg, t_ok, sx, sy, sg, s_ok, u, v, ru, rv);
-}
-
 // The sources of a tile in the warp's shared buffer, each twice, 32 entries apart, so that step k of
 // lane l reads entry l + k without a wrap.
 struct SourceBuffer {
     double2 xy[64];
     double g[64];
-    __device__ __forceinline__ void fill(double sx, double sy, double sg) {
+    __device__ __forceinline__ void fill(const Vortex &s) {
         const int lane = threadIdx.x & 31;
         __syncwarp();  // the previous tile's reads are done
-        xy[lane] = xy[lane + 32] = make_double2(sx, sy);
-        g[lane] = g[lane + 32] = sg;
+        xy[lane] = xy[lane + 32] = make_double2(s.x, s.y);
+        g[lane] = g[lane + 32] = s.g;
         __syncwarp();
     }
 };
@@ -135,31 +217,21 @@ struct SourceBuffer {
 // and source present. Only the reactions rotate (two double shuffles a step, shared by the T
 // pairs); reading the sources instead of rotating them too (five) is 6 % faster with the box's
 // terms (N = 16384, T = 1: 500 against 532 us; T = 2: 472 against 493 us). U steps are unrolled:
-// two with one target per lane, four with two.
-template <class P, int T, bool NEAR, int U = (T == 2 ? 4 : 2)>
-__device__ __forceinline__ void react_tiles_steps(const GeometryConsts &g, const double (&tx)[T],
-                                                 const double (&ty)[T], const double (&tg)[T],
-                                                 const SourceBuffer &b, double (&u)[T],
-                                                 double (&v)[T], double &ru, double &rv) {
+// two with one target per lane, four with two, none with four (the disk at N = 16384: 314 against
+// 325 us unrolled by two).
+template <class P, int T, bool NEAR, int U = (T == 2 ? 4 : T == 4 ? 1 : 2)>
+__device__ __forceinline__ void react_tiles_steps(const GeometryConsts &g, const Vortex (&t)[T],
+                                                  const SourceBuffer &b, double (&u)[T],
+                                                  double (&v)[T], double &ru, double &rv) {
     const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
     const double2 *xy = b.xy + lane;
     const double *sgs = b.g + lane;
 #pragma unroll U
     for (int k = 0; k < 32; ++k) {
-        const double2 s = xy[k];
-        const double sg = sgs[k];
+        const Vortex s = {xy[k].x, xy[k].y, sgs[k]};
 #pragma unroll
-        for (int t = 0; t < T; ++t) {
-            double ku, kv;
-            if constexpr (NEAR)
-                P::values_near(g, tx[t], ty[t], s.x, s.y, ku, kv);
-            else
-                P::values(g, tx[t], ty[t], s.x, s.y, ku, kv);
-            u[t] = fma(-sg, ku, u[t]);    // target: -c_s K
-            v[t] = fma(sg, kv, v[t]);
-            ru = fma(tg[t], ku, ru);      // source: the exchanged pair, +c_t K
-            rv = fma(-tg[t], kv, rv);
-        }
+        for (int q = 0; q < T; ++q)
+            P::template react<NEAR>(g, t[q], s, u[q], v[q], ru, rv);
         ru = rotate(ru, next);
         rv = rotate(rv, next);
     }
@@ -171,25 +243,18 @@ __device__ __forceinline__ void react_tiles_steps(const GeometryConsts &g, const
 // 1892 us at 65 536.
 template <class P, int T>
 __device__ __forceinline__ void react_tiles_rotating(const GeometryConsts &g,
-                                                     const double (&tx)[T], const double (&ty)[T],
-                                                     const double (&tg)[T], double sx, double sy,
-                                                     double sg, double (&u)[T], double (&v)[T],
-                                                     double &ru, double &rv) {
+                                                     const Vortex (&t)[T], Vortex s,
+                                                     double (&u)[T], double (&v)[T], double &ru,
+                                                     double &rv) {
     const int next = (threadIdx.x + 1) & 31;
 #pragma unroll 2
     for (int k = 0; k < 32; ++k) {
 #pragma unroll
-        for (int t = 0; t < T; ++t) {
-            double ku, kv;
-            P::values(g, tx[t], ty[t], sx, sy, ku, kv);
-            u[t] = fma(-sg, ku, u[t]);
-            v[t] = fma(sg, kv, v[t]);
-            ru = fma(tg[t], ku, ru);
-            rv = fma(-tg[t], kv, rv);
-        }
-        sx = rotate(sx, next);
-        sy = rotate(sy, next);
-        sg = rotate(sg, next);
+        for (int q = 0; q < T; ++q)
+            P::template react<false>(g, t[q], s, u[q], v[q], ru, rv);
+        s.x = rotate(s.x, next);
+        s.y = rotate(s.y, next);
+        s.g = rotate(s.g, next);
         ru = rotate(ru, next);
         rv = rotate(rv, next);
     }
@@ -197,44 +262,41 @@ __device__ __forceinline__ void react_tiles_rotating(const GeometryConsts &g,
 
 // One whole tile set of T targets per lane. near: this lane's targets satisfy P::near.
 template <class P, int T, bool BUFFERED>
-__device__ __forceinline__ void react_tiles_full(const GeometryConsts &g, const double (&tx)[T],
-                                                 const double (&ty)[T], const double (&tg)[T],
-                                                 double sx, double sy, double sg, SourceBuffer &b,
-                                                 bool near, double (&u)[T], double (&v)[T],
-                                                 double &ru, double &rv) {
+__device__ __forceinline__ void react_tiles_full(const GeometryConsts &g, const Vortex (&t)[T],
+                                                 const Vortex &s, SourceBuffer &b, bool near,
+                                                 double (&u)[T], double (&v)[T], double &ru,
+                                                 double &rv) {
     if constexpr (!BUFFERED) {
-        react_tiles_rotating<P, T>(g, tx, ty, tg, sx, sy, sg, u, v, ru, rv);
+        react_tiles_rotating<P, T>(g, t, s, u, v, ru, rv);
         return;
     }
-    b.fill(sx, sy, sg);
+    b.fill(s);
     if constexpr (P::kNearForm) {
-        if (__all_sync(0xffffffffu, near && P::near(g, sx, sy))) {
-            react_tiles_steps<P, T, true>(g, tx, ty, tg, b, u, v, ru, rv);
+        if (__all_sync(0xffffffffu, near && P::near(g, s.x, s.y))) {
+            react_tiles_steps<P, T, true>(g, t, b, u, v, ru, rv);
             return;
         }
     }
-    react_tiles_steps<P, T, false>(g, tx, ty, tg, b, u, v, ru, rv);
+    react_tiles_steps<P, T, false>(g, t, b, u, v, ru, rv);
 }
 
-// Target side only. same_block: the sources are the targets' own lanes, so the self pair (k = 0)
-// is skipped; the reference skips it too (and in the periodic box it contributes exactly 0).
-template <class P = PeriodicSym>
-__device__ __forceinline__ void one_sided_tile(const GeometryConsts &g, double tx, double ty,
-                                               bool t_ok, double sx, double sy, double sg,
-                                               int s_ok, bool same_block, double &u, double &v) {
+// Target side only. same_block: the sources are the targets' own lanes, so step 0 is the vortex
+// itself.
+template <class P>
+__device__ __forceinline__ void one_sided_tile(const GeometryConsts &g, const Vortex &t, bool t_ok,
+                                               Vortex s, int s_ok, bool same_block, double &u,
+                                               double &v) {
     const int next = (threadIdx.x + 1) & 31;
     for (int k = 0; k < 32; ++k) {
-        if (t_ok && s_ok && !(same_block && k == 0)) {
-            double ku, kv;
-            P::values(g, tx, ty, sx, sy, ku, kv);
-            u = fma(-sg, ku, u);
-            v = fma(sg, kv, v);
-        }
-        sx = rotate(sx, next);
-        sy = rotate(sy, next);
-        sg = rotate(sg, next);
+        if (t_ok && s_ok && !(same_block && k == 0))
+            P::one(g, t, s, u, v);
+        s.x = rotate(s.x, next);
+        s.y = rotate(s.y, next);
+        s.g = rotate(s.g, next);
         s_ok = __shfl_sync(0xffffffffu, s_ok, next);
     }
+    if (same_block && t_ok)
+        P::self(g, t, u, v);
 }
 
 // FP32-compensated tiles: the 32 sources (hi/lo coordinates and FP32 circulation) sit in this
