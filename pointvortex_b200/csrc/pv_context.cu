@@ -367,6 +367,11 @@ pv_status make_consts(const pv_params &p, GeometryConsts &g, std::string &messag
                 if (k < 3)
                     g.zq[k] = static_cast<double>(kZetaQ[k] * power / lead);
             }
+            power = 1.0L;
+            for (int k = 0; k < 8; ++k, power *= unit4)
+                g.zs[k] = static_cast<double>(kZetaS[k] * power);
+            g.energy_r2 = static_cast<double>(-kPiLong / lx / lx);
+            g.energy_0 = static_cast<double>(kEnergyConstant + 2.0L * std::log(2.0L * kPiLong / lx));
         }
         return PV_OK;
     }

@@ -87,3 +87,25 @@ def test_exchange_negates_the_term_exactly():
     x, y = _points(2 * np.pi)
     a, b = _term(x, y, 2 * np.pi), _term(-x, -y, 2 * np.pi)
     assert np.array_equal(a[0], -b[0]) and np.array_equal(a[1], -b[1])
+
+
+def test_energy_matches_the_image_logarithms():
+    """box_energy against the reference's sum (src/compute.cpp:186-196), both in extended precision:
+    what is checked are the coefficients, good to 8.8e-19 of sigma and rounded to double, so within
+    2 * 2^-53 per coefficient's share (below 1.2 in sum) of the logarithm."""
+    s = _coefficients("kZetaS")
+    e0 = LD(re.search(r"kEnergyConstant = ([-0-9.]+);", HEADER.read_text()).group(1))
+    for length in (2 * np.pi, 0.3):
+        x, y = _points(length)
+        x, y = x.astype(LD), y.astype(LD)
+        w = ((x + 1j * y) * 2 / LD(length)) ** 4
+        poly = sum(LD(c) * w ** k for k, c in enumerate(s))
+        r = x * x + y * y
+        got = e0 + 2 * np.log(2 * PI / LD(length)) - PI * r / LD(length) ** 2 + np.log(r * abs(poly) ** 2)
+        hx, hy = 2 * PI / LD(length) * x, 2 * PI / LD(length) * y
+        want = -hx * hx / (2 * PI) + np.log(2 * (np.sinh(hx / 2) ** 2 + np.sin(hy / 2) ** 2))
+        for m in range(1, 9):
+            a = 2 * PI * m
+            # (cosh(x - a) - cos y)(cosh(x + a) - cos y) / cosh^2 a
+            want += np.log((np.cosh(hx) / np.cosh(a) - np.cos(hy)) ** 2 + (np.tanh(a) * np.sin(hy)) ** 2)
+        assert np.max(np.abs(got - want)) <= 4 * 2.0 ** -53

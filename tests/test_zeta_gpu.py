@@ -60,3 +60,18 @@ def test_symmetric_tiles(port, n, targets):
         check(port, 2.0, 8, x, y, g, device_state=True)
     finally:
         autotune.set_symmetric_entry(1, 0, 11, *saved)
+
+
+@pytest.mark.parametrize("layers", [5, 6, 64])
+@pytest.mark.parametrize("length", [1.0 / 65536.0, 2.0, 7e4])
+@pytest.mark.parametrize("n", [2, 128, 130, 386])
+def test_hamiltonian_routes(port, layers, length, n):
+    """The sigma form and the image product on both sides of the rule, tiles whole and ragged,
+    positions outside the box; the Hamiltonian's parity tolerance (1e-12 of its terms' scale)."""
+    x, y, g = ics.periodic_box(n, 11 + n, length)
+    x[::3] += 3 * length
+    k = pv.PeriodicBoxKernel(length, length, layers)
+    got = k.invariants(pv.VortexSystem(x, y, g)).hamiltonian
+    geo = Geometry("periodic", box_length_x=length, box_length_y=length, image_layers=layers)
+    want = port.invariants(geo, x, y, g)[4]
+    assert abs(got - want) <= 1e-12 * max(abs(want), 1.0)
