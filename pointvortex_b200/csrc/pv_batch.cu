@@ -7,12 +7,12 @@
 //
 //   * velocity: a persistent grid (one wave of resident CTAs) drains a work queue of
 //     (simulation, block of 128 threads x T targets, chunk of sources) items with an atomic counter. The
-//     items are sorted by cost (periodic pairs cost ~15x plane pairs), so the longest go first.
+//     items are sorted by cost (a pair of the box costs 5-12 plane pairs), so the longest go first.
 //     Each CTA copies the item's geometry constants to shared memory and runs the same TMA-staged
-//     tile loop and pair functions as the single-simulation kernel. Periodic simulations (both
-//     forms) from N = 2048 instead take (simulation, block I, block J) items of 128 x 128 evaluated once
-//     per unordered pair (the warp tiles of pv_symmetric.cuh, reactions summed across the CTA's
-//     warps in fixed order). Simulations in the FP32-compensated form drain a second queue, in a
+//     tile loop and pair functions as the single-simulation kernel. Periodic and disk simulations
+//     (batch_pair_items) instead take (simulation, block I, block J) items of 128 x 128 evaluated
+//     once per unordered pair (the warp tiles of pv_symmetric.cuh, reactions summed across the
+//     CTA's warps in fixed order). Simulations in the FP32-compensated form drain a second queue, in a
 //     second launch, with the pair terms of pv_pair32.cuh;
 //   * stage: one 256-element block per slice of a simulation reduces that simulation's chunk
 //     partials in fixed order, then forms the next stage position or the DOPRI5 error;
@@ -62,12 +62,42 @@ constexpr bool batch_targets_allowed(int geometry, int per_thread) {
 // Atomic entries: a table update may run beside admissions on other host threads.
 std::atomic<int> g_batch_tuning[3][2][40] = {};
 
-int batch_targets_for(int geometry, int precision, size_t n) {
+int batch_entry(int geometry, int precision, size_t n) {
     int bucket = 0;
     while ((size_t(2) << bucket) <= n && bucket < 39)
         ++bucket;
-    const int t = g_batch_tuning[geometry][precision][bucket].load(std::memory_order_relaxed);
+    return g_batch_tuning[geometry][precision][bucket].load(std::memory_order_relaxed);
+}
+
+int batch_targets_for(int geometry, int precision, size_t n) {
+    const int t = batch_entry(geometry, precision, n);
     return t ? t : default_targets_per_thread(geometry);
+}
+
+// Once-per-unordered-pair items (128 x 128 block pairs, a partial row a block) or ordered items:
+// a function of the simulation's own geometry, precision and population and of the tables.
+//   * the periodic box from kSymmetricMinN up, both forms, unless its table
+//     (pv_set_symmetric_tuning) says otherwise;
+//   * FP64, the box and the disk from one whole block up to kPairRowsMaxN, where the batch table has
+//     no entry (an entry asks for ordered items). Their pairs cost less than half there (box 50 FP64
+//     instructions against 98 for the two ordered pairs, disk 34 against 58), and the items are a
+//     quarter of an ordered item's (128 x 512), so the queue's last round is fuller. 96 members of
+//     64 to 4096 vortices, geometries in turn: 3.40 ms an attempt with ordered items and
+//     PeriodicPair, 1.88 ms now. The plane's (13 against 20) would be bound by the tile's shuffles
+//     and shared loads;
+//   * kPairRowsMaxN bounds the partial rows of these smaller members: kPairRows a vortex, which the
+//     arena holds beside the caller's own (pv_batch_create), so no admission is refused for them.
+constexpr size_t kPairRows = 32;
+constexpr size_t kPairRowsMaxN = kPairRows * 128;
+bool batch_pair_items(const GeometryConsts &g, int precision, size_t n) {
+    if (n < 128)
+        return false;
+    const int tuned = symmetric_tuning_lookup(g.geometry, precision, n) & 15;
+    if (g.geometry == GEO_PERIODIC && (tuned == 2 || (tuned == 0 && n >= kSymmetricMinN)))
+        return true;
+    return precision == PV_PRECISION_FP64 && n <= kPairRowsMaxN && tuned == 0 &&
+           (g.geometry == GEO_DISK || (g.geometry == GEO_PERIODIC && g.zeta)) &&
+           batch_entry(g.geometry, precision, n) == 0;
 }
 // Sources per work item, a function of the population only (so a simulation's summation order
 // never depends on its batch): 512 up to N = 16384, then N/32 rounded up to 512.
@@ -84,7 +114,7 @@ struct SimDesc {
     unsigned num_chunks;          // partial rows (chunks, or 128-blocks of the symmetric form)
     unsigned chunk;
     int precision;                // PV_PRECISION_*
-    int symmetric;                // periodic, evaluated once per unordered pair (either form)
+    int symmetric;                // evaluated once per unordered pair (batch_pair_items)
     int per_thread;               // targets per thread of the ordered items (1, 2 or 4)
 };
 
@@ -243,15 +273,17 @@ __device__ __forceinline__ void run_item(const GeometryConsts &g, const double *
         }
 }
 
-// One 128 x 128 block pair of a periodic FP64 simulation, once per unordered pair: warp w holds
-// targets I*128 + 32w + lane and meets the four 32-source sub-tiles of block J in turn. Targets'
-// sums go to row J, the sources' reactions (summed over the four warps in fixed order) to row I.
-// A diagonal item (I == J) is evaluated one-sided. red_u / red_v: 4 x 128 doubles of shared memory.
+// One 128 x 128 block pair of an FP64 simulation, once per unordered pair: warp w holds targets
+// I*128 + 32w + lane and meets the four 32-source sub-tiles of block J in turn. Targets' sums go to
+// row J, the sources' reactions (summed over the four warps in fixed order) to row I. A diagonal
+// item (I == J) is evaluated one-sided. red_u / red_v: 4 x 128 doubles of shared memory; src: the
+// warp's source buffer.
 template <class P>
 __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, const double *px,
                                                    const double *py, const double *sgs, size_t n,
                                                    unsigned I, unsigned J, double *pu, double *pv,
-                                                   size_t pad_n, double *red_u, double *red_v) {
+                                                   size_t pad_n, double *red_u, double *red_v,
+                                                   sym::SourceBuffer &src) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool diagonal = I == J;
     const size_t ti = static_cast<size_t>(I) * kBlock + static_cast<size_t>(w) * 32 + lane;
@@ -270,10 +302,16 @@ __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, cons
             sym::one_sided_tile<P>(g, t, t_ok, s, s_ok, q == w, u, v);
         } else {
             double ru = 0.0, rv = 0.0;
-            if (__all_sync(0xffffffffu, t_ok && s_ok))
-                sym::react_tile_t<P, true>(g, t, t_ok, s, s_ok, u, v, ru, rv);
-            else
+            if (__all_sync(0xffffffffu, t_ok && s_ok)) {
+                const sym::Vortex t1[1] = {t};
+                double u1[1] = {u}, v1[1] = {v};
+                sym::react_tiles_full<P, 1, true>(g, t1, s, src, P::near(g, t.x, t.y), u1, v1, ru,
+                                                  rv);
+                u = u1[0];
+                v = v1[0];
+            } else {
                 sym::react_tile_t<P, false>(g, t, t_ok, s, s_ok, u, v, ru, rv);
+            }
             red_u[w * kBlock + q * 32 + lane] = ru;
             red_v[w * kBlock + q * 32 + lane] = rv;
         }
@@ -548,6 +586,7 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
     __shared__ alignas(8) float s_gf[PREC == PV_PRECISION_FP32C ? 2 * kTileB : 1];  // disk: (g, -g)
     __shared__ alignas(8) uint64_t bars[2];
     __shared__ GeometryConsts s_geo;
+    __shared__ sym::SourceBuffer s_src[PREC == PV_PRECISION_FP64 ? kBlock / 32 : 1];
     __shared__ unsigned s_item;
     if (threadIdx.x == 0) {
         mbar_init(&bars[0], 1);
@@ -588,9 +627,20 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
             if constexpr (PREC == PV_PRECISION_FP32C)
                 run_symmetric_item32(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu, pv, d.pad_n,
                                      &s_x[0][0], &s_y[0][0], s_f, s_gf);
-            else
-                run_symmetric_item<sym::PeriodicSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu, pv, d.pad_n,
-                                   &s_x[0][0], &s_y[0][0]);
+            else {
+                sym::SourceBuffer &src = s_src[threadIdx.x >> 5];
+                if (s_geo.geometry == GEO_DISK)
+                    run_symmetric_item<sym::DiskSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu,
+                                                     pv, d.pad_n, &s_x[0][0], &s_y[0][0], src);
+                else if (s_geo.zeta)
+                    run_symmetric_item<sym::ZetaUnitSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk,
+                                                         pu, pv, d.pad_n, &s_x[0][0], &s_y[0][0],
+                                                         src);
+                else
+                    run_symmetric_item<sym::PeriodicSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk,
+                                                         pu, pv, d.pad_n, &s_x[0][0], &s_y[0][0],
+                                                         src);
+            }
             __syncthreads();
             continue;
         }
@@ -601,6 +651,8 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
         const size_t blk1 = min(blk0 + per_block, static_cast<size_t>(d.n));
         const size_t out0 = static_cast<size_t>(it.chunk) * d.pad_n;
         // one instantiation per (geometry, targets per thread) the batch table allows
+        // (FP64: the box from six images up counts as a geometry of its own, GEO_ZETA)
+        constexpr int GEO_ZETA = 3;
         auto ordered = [&](auto geo, auto per_thread) {
             constexpr int G = decltype(geo)::value, T = decltype(per_thread)::value;
             if constexpr (PREC == PV_PRECISION_FP32C) {
@@ -608,7 +660,8 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
                                  s_g, s_f, s_fi, s_gf, bars, seq, a.timeout_status, timed_out);
             } else {
                 using Pair = std::conditional_t<G == GEO_INFINITE, InfinitePair,
-                             std::conditional_t<G == GEO_PERIODIC, PeriodicPair, DiskPair>>;
+                             std::conditional_t<G == GEO_PERIODIC, PeriodicPair,
+                             std::conditional_t<G == GEO_ZETA, ZetaUnitPair, DiskPair>>>;
                 run_item<Pair, T>(s_geo, px, py, sgs, src0, src1, blk0, blk1, pu, pv, out0, s_x,
                                   s_y, s_g, bars, seq, a.timeout_status, timed_out);
             }
@@ -616,15 +669,19 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
         using I0 = std::integral_constant<int, GEO_INFINITE>;
         using I1 = std::integral_constant<int, GEO_PERIODIC>;
         using I2 = std::integral_constant<int, GEO_DISK>;
+        using I3 = std::integral_constant<int, PREC == PV_PRECISION_FP64 ? GEO_ZETA : GEO_PERIODIC>;
         using T1 = std::integral_constant<int, 1>;
         using T2 = std::integral_constant<int, 2>;
         using T4 = std::integral_constant<int, 4>;
-        switch (s_geo.geometry * 8 + d.per_thread) {
+        const int form = PREC == PV_PRECISION_FP64 && s_geo.zeta ? GEO_ZETA : s_geo.geometry;
+        switch (form * 8 + d.per_thread) {
         case GEO_INFINITE * 8 + 1: ordered(I0{}, T1{}); break;
         case GEO_INFINITE * 8 + 2: ordered(I0{}, T2{}); break;
         case GEO_INFINITE * 8 + 4: ordered(I0{}, T4{}); break;
         case GEO_PERIODIC * 8 + 1: ordered(I1{}, T1{}); break;
         case GEO_PERIODIC * 8 + 2: ordered(I1{}, T2{}); break;
+        case GEO_ZETA * 8 + 1: ordered(I3{}, T1{}); break;
+        case GEO_ZETA * 8 + 2: ordered(I3{}, T2{}); break;
         case GEO_DISK * 8 + 1: ordered(I2{}, T1{}); break;
         case GEO_DISK * 8 + 2: ordered(I2{}, T2{}); break;
         default: ordered(I2{}, T4{}); break;  // admission allows no other combination
@@ -965,7 +1022,10 @@ pv_status rebuild_tables(pv_batch *b) {
             continue;
         const SimDesc &d = b->descs[s];
         const int q = d.precision == PV_PRECISION_FP32C ? 1 : 0;
-        const double w = d.g.geometry == GEO_PERIODIC ? 15.0 : (d.g.geometry == GEO_DISK ? 2.7 : 1.0);
+        // a pair's cost in an item of its form: FP64 pipe cycles over the plane's ordered pair's 22
+        const double w = d.g.geometry == GEO_PERIODIC ? (d.g.zeta && q == 0 ? 5.5 : 12.0)
+                         : d.g.geometry == GEO_DISK   ? (d.symmetric ? 3.5 : 3.0)
+                                                      : 1.0;
         if (d.symmetric) {
             const unsigned nb = symmetric_rows(d.n);
             for (unsigned I = 0; I < nb; ++I)
@@ -1173,7 +1233,7 @@ pv_status pv_batch_create(const pv_batch_config *config, pv_batch **out) {
     // partials: each simulation needs ceil(n/512) chunks of pad(n); bounded by capacity^2/512 but
     // allocated as a multiple of the element capacity (sized by the caller's partial factor)
     const size_t factor = config->partial_chunks_per_vortex_slot ? config->partial_chunks_per_vortex_slot : 16;
-    b->part_capacity = b->capacity * factor;
+    b->part_capacity = b->capacity * (factor + kPairRows);
     const size_t arrays = 4 + 4 + 14;
     const size_t bytes = (arrays * b->capacity + 2 * b->part_capacity) * sizeof(double);
     if ((e = cudaMalloc(&b->arena_block, bytes)) != cudaSuccess)
@@ -1272,13 +1332,7 @@ pv_status pv_batch_add(pv_batch *b, const pv_params *params, const double *x, co
         return bfail(b, PV_ERROR_INVALID_ARGUMENT, "unknown precision form");
     const size_t pad = round_up(n, kAlign);
     const size_t chunk = chunk_for(n);
-    // periodic populations from kSymmetricMinN up: once per unordered pair, one partial row
-    // per 128-block. The autotuner's table of the symmetric form (pv_set_symmetric_tuning) may
-    // choose otherwise for the population's size; either way the choice is a function of the
-    // simulation's own n, geometry and precision, never of the batch.
-    const int tuned = symmetric_tuning_lookup(g.geometry, params->precision, n) & 15;
-    const bool symmetric = g.geometry == GEO_PERIODIC && n >= 128 &&
-                           (tuned == 2 || (tuned == 0 && n >= kSymmetricMinN));
+    const bool symmetric = batch_pair_items(g, params->precision, n);
     const unsigned chunks = symmetric ? symmetric_rows(static_cast<unsigned>(n))
                                       : static_cast<unsigned>((n + chunk - 1) / chunk);
     size_t off = 0, poff = 0;

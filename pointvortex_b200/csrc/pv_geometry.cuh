@@ -251,6 +251,22 @@ constexpr double kZetaP[6] = {0.99999999999999999987, -0.24693625978040467126,
 constexpr double kZetaQ[4] = {1.0, -0.04998550964578607478, -0.00083074426019041809798,
                               3.0367890005030402872e-06};
 
+// The same function in units of L/2 with a monic denominator: kZetaP (2/pi) / kZetaQ[3] and
+// kZetaQ / kZetaQ[3]. With these the coefficients are literals (UNIT below).
+__host__ __device__ constexpr double zeta_unit_p(int k) {
+    return k == 0   ? 2.0963582661229544646e+5
+           : k == 1 ? -5.1766686939613659311e+4
+           : k == 2 ? -1.5953651295191684159e+3
+           : k == 3 ? 7.5435808913963043333
+           : k == 4 ? 1.1245010326330765775e-3
+                    : 5.3805505458809630715e-5;
+}
+__host__ __device__ constexpr double zeta_unit_q(int k) {
+    return k == 0   ? 3.2929518640720552362e+5
+           : k == 1 ? -1.6459987716468295239e+4
+                    : -2.7356008601611977445e+2;
+}
+
 // sigma(z)/z as a polynomial in z^4 over the box (relative error 8.8e-19, fitted as kZetaP), and the
 // constant of box_energy in units of the reduced displacement (2 pi/L) z.
 constexpr double kZetaS[8] = {1.0, -4.9237687533654649034e-2, -8.6583924059350373423e-4,
@@ -265,28 +281,43 @@ __device__ __forceinline__ double exponent_up(double v, int powers) {
     return __hiloint2double(__double2hiint(v) + (powers << 20), __double2loint(v));
 }
 
-struct ZetaPair {
+// UNIT: the coefficients as literals for displacements in units of L/2, at two multiplications a
+// pair. For kernels whose GeometryConsts is not a kernel parameter (the ensembles': one box after
+// another), where each coefficient would be a load from shared memory for every pair.
+template <bool UNIT> struct ZetaPairT {
     // The kernel values of a reduced displacement.
     __device__ __forceinline__ static void terms(const GeometryConsts &g, double x, double y,
                                                  double &ku, double &kv) {
+        double zp[6], zq[3];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            zp[k] = UNIT ? zeta_unit_p(k) : g.zp[k];
+            if (k < 3)
+                zq[k] = UNIT ? zeta_unit_q(k) : g.zq[k];
+        }
+        if (UNIT) {
+            x *= 2.0 * g.inv_lx;
+            y *= 2.0 * g.inv_lx;
+        }
+        const double linear = UNIT ? 0.5 : g.inv_lx;
         const double yy = y * y;
         const double a = fma(x, x, -yy), r = fma(x, x, yy), b = x * y;  // z^2 = a + 2ib, r = |z|^2
         const double r2 = r * r, n = r2 * r2;                           // |w|^2, w = z^4
         const double wr = fma(-8.0 * b, b, r2);
         const double wi = exponent_up(a * b, 2);
         const double tr = exponent_up(wr, 1);
-        const double p4 = fma(tr, g.zp[5], g.zp[4]);
-        const double p3 = fma(tr, p4, fma(-n, g.zp[5], g.zp[3]));
-        const double p2 = fma(tr, p3, fma(-n, p4, g.zp[2]));
-        const double p1 = fma(tr, p2, fma(-n, p3, g.zp[1]));
-        const double pr = fma(wr, p1, fma(-n, p2, g.zp[0])), pi = wi * p1;
-        const double q2 = tr + g.zq[2];
-        const double q1 = fma(tr, q2, g.zq[1] - n);
-        const double qr = fma(wr, q1, fma(-n, q2, g.zq[0])), qi = wi * q1;
+        const double p4 = fma(tr, zp[5], zp[4]);
+        const double p3 = fma(tr, p4, fma(-n, zp[5], zp[3]));
+        const double p2 = fma(tr, p3, fma(-n, p4, zp[2]));
+        const double p1 = fma(tr, p2, fma(-n, p3, zp[1]));
+        const double pr = fma(wr, p1, fma(-n, p2, zp[0])), pi = wi * p1;
+        const double q2 = tr + zq[2];
+        const double q1 = fma(tr, q2, zq[1] - n);
+        const double qr = fma(wr, q1, fma(-n, q2, zq[0])), qi = wi * q1;
         const double dr = fma(x, qr, -y * qi), di = fma(x, qi, y * qr);  // z Q
         const double inv = rcp_refined(fma(dr, dr, di * di));
-        ku = fma(fma(pr, di, -pi * dr), inv, -g.inv_lx * y);
-        kv = fma(fma(pr, dr, pi * di), inv, -g.inv_lx * x);
+        ku = fma(fma(pr, di, -pi * dr), inv, -linear * y);
+        kv = fma(fma(pr, dr, pi * di), inv, -linear * x);
     }
 
     // remainder(d, L) for |d| <= 3L/2: one subtraction of 0 or +-L (exact, as the remainder is),
@@ -329,6 +360,8 @@ struct ZetaPair {
         v = fma(sg, kv, v);
     }
 };
+using ZetaPair = ZetaPairT<false>;
+using ZetaUnitPair = ZetaPairT<true>;
 
 // The box's pair energy in the same units, -x^2/(2 pi) + sum_m [log D(m) - log cosh(2 pi m)] of the
 // reference (x, y here times 2 pi/L), which is 2 log|sigma(z)| - pi |z|^2/L^2 + constant: sigma is

@@ -79,23 +79,24 @@ struct PeriodicSym : Antisymmetric<PeriodicSym> {
 // The box from six images up (ZetaPair). Tiles whose vortices are all in or near the box reduce a
 // difference by one subtraction (values_near): two FP64 instructions an axis with it, four without
 // (a population that has drifted out of the box: 8 % more of the pair's 50).
-struct ZetaSym : Antisymmetric<ZetaSym> {
+template <class Z> struct ZetaSymT : Antisymmetric<ZetaSymT<Z>> {
     static constexpr bool kNearForm = true;
     __device__ __forceinline__ static void values(const GeometryConsts &g, double tx, double ty,
                                                   double sx, double sy, double &ku, double &kv) {
-        ZetaPair::terms(g, ZetaPair::reduce(g, tx - sx, g.lx, g.inv_lx),
-                        ZetaPair::reduce(g, ty - sy, g.ly, g.inv_ly), ku, kv);
+        Z::terms(g, Z::reduce(g, tx - sx, g.lx, g.inv_lx), Z::reduce(g, ty - sy, g.ly, g.inv_ly), ku,
+                 kv);
     }
     __device__ __forceinline__ static void values_near(const GeometryConsts &g, double tx,
                                                        double ty, double sx, double sy,
                                                        double &ku, double &kv) {
-        ZetaPair::terms(g, ZetaPair::reduce_near(g, tx - sx, g.lx),
-                        ZetaPair::reduce_near(g, ty - sy, g.ly), ku, kv);
+        Z::terms(g, Z::reduce_near(g, tx - sx, g.lx), Z::reduce_near(g, ty - sy, g.ly), ku, kv);
     }
     __device__ __forceinline__ static bool near(const GeometryConsts &g, double x, double y) {
-        return ZetaPair::inside(g, x, y);
+        return Z::inside(g, x, y);
     }
 };
+using ZetaSym = ZetaSymT<ZetaPair>;
+using ZetaUnitSym = ZetaSymT<ZetaUnitPair>;
 
 // The infinite plane (InfinitePair): K = (dy, dx) / (r^2 + eps^2), exactly odd in (dx, dy).
 struct PlaneSym : Antisymmetric<PlaneSym> {
