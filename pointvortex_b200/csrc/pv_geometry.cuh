@@ -363,6 +363,17 @@ template <bool UNIT> struct ZetaPairT {
 using ZetaPair = ZetaPairT<false>;
 using ZetaUnitPair = ZetaPairT<true>;
 
+// One ordered pair of the box, by the form its constants allow.
+template <bool CHECK>
+__device__ __forceinline__ void periodic_pair(const GeometryConsts &g, double tx, double ty,
+                                              double sx, double sy, double sg, bool self, double &u,
+                                              double &v) {
+    if (g.zeta)
+        ZetaPair::pair<CHECK>(g, tx, ty, sx, sy, sg, self, u, v);
+    else
+        PeriodicPair::pair<CHECK>(g, tx, ty, sx, sy, sg, self, u, v);
+}
+
 // The box's pair energy in the same units, -x^2/(2 pi) + sum_m [log D(m) - log cosh(2 pi m)] of the
 // reference (x, y here times 2 pi/L), which is 2 log|sigma(z)| - pi |z|^2/L^2 + constant: sigma is
 // entire, sigma(z)/z a function of z^4 alone, and a polynomial of degree 7 over the box. One logarithm

@@ -65,7 +65,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 4) near_field_kernel(const Ne
         // are dropped
         for (size_t j = lane; j < a.n; j += 32) {
             if (a.g.geometry == GEO_PERIODIC)
-                PeriodicPair::pair<true>(a.g, tx, ty, a.x[j], a.y[j], a.gs[j], j == i, du, dv);
+                periodic_pair<true>(a.g, tx, ty, a.x[j], a.y[j], a.gs[j], j == i, du, dv);
             else
                 DiskPair::pair<true>(a.g, tx, ty, a.x[j], a.y[j], a.gs[j], j == i, du, dv);
         }
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(kNearWarps * 32, 4) near_field_kernel(const Ne
         if (key & 1u)
             DiskPair::image(a.g, tx, ty, a.x[j], a.y[j], a.gs[j], du, dv);
         else if (a.g.geometry == GEO_PERIODIC)
-            PeriodicPair::pair<false>(a.g, tx, ty, a.x[j], a.y[j], a.gs[j], false, du, dv);
+            periodic_pair<false>(a.g, tx, ty, a.x[j], a.y[j], a.gs[j], false, du, dv);
         else
             DiskPair::direct(tx, ty, a.x[j], a.y[j], a.gs[j], du, dv);
     }

@@ -56,6 +56,8 @@ struct F32Geometry { // the FP32 constants of one evaluation
     int m_exact;
     float inv_radius2;
     float near2;       // near-field radius squared (0: no near field)
+    float unit;        // 2/L
+    float near2_unit;  // near2 in units of L/2
 };
 
 __device__ __forceinline__ F32Geometry make_f32(const GeometryConsts &g) {
@@ -79,6 +81,8 @@ __device__ __forceinline__ F32Geometry make_f32(const GeometryConsts &g) {
     f.m_exact = g.m_exact;
     f.inv_radius2 = static_cast<float>(g.inv_radius2);
     f.near2 = static_cast<float>(g.near2);
+    f.unit = static_cast<float>(2.0 * g.inv_lx);
+    f.near2_unit = static_cast<float>(4.0 * g.near2 * g.inv_lx * g.inv_lx);
     return f;
 }
 
@@ -202,6 +206,57 @@ __device__ __forceinline__ bool periodic_values32(const F32Geometry &f, const fl
     return near;
 }
 
+// The periodic pair's kernel values from six images up, two pairs at a time (one in each f32x2
+// lane): the rational form of ZetaPair (pv_geometry.cuh) at FP32 accuracy, P of degree 3 over a monic
+// Q of degree 2 in z^4 (relative error 2.5e-9 over the box, fitted alike), displacements in units
+// of L/2. th, tl: the target's hi and lo coordinates splat over the lanes; nsh, nsl: the two
+// sources', negated. Exactly odd under exchanging target and source. near: which lanes' pairs lie
+// closer than the near-field radius; their values come back as 0.
+//
+// 59 f32x2 instructions for two pairs, where periodic_core_x2 packs the two axes of one pair into
+// about as many. Per launch, that form against this: N = 4096 50 -> 36 us, 16 384 507 -> 313 us, 65 536
+// 7.77 -> 4.65 ms; rms error of a velocity 4-11 % lower. Bound by register reads: an f32x2
+// instruction with three distinct operands takes three cycles, and the scalar form (one cycle each)
+// issues too much: 344 us at N = 16 384.
+__device__ __forceinline__ void zeta_values32_x2(const F32Geometry &f, float2 thx, float2 thy,
+                                                 float2 tlx, float2 tly, float2 nshx, float2 nshy,
+                                                 float2 nslx, float2 nsly, float2 &ku, float2 &kv,
+                                                 bool &near0, bool &near1) {
+    const float kP0 = -662.991228f, kP1 = 161.815890f, kP2 = 5.50566322f, kP3 = -0.00715411985f;
+    const float kQ0 = -1041.42419f, kQ1 = 49.0705318f;
+    const float2 dx = add2(add2(thx, nshx), add2(tlx, nslx));
+    const float2 dy = add2(add2(thy, nshy), add2(tly, nsly));
+    // remainder(d, L): rounding to an integer by adding and taking off 1.5 2^23
+    const float2 big = splat2(12582912.0f), nbig = splat2(-12582912.0f);
+    const float2 nx = add2(fma2(dx, splat2(f.inv_l), big), nbig);
+    const float2 ny = add2(fma2(dy, splat2(f.inv_l), big), nbig);
+    const float2 rx = fma2(nx, splat2(-f.l_lo), fma2(nx, splat2(-f.l_hi), dx));
+    const float2 ry = fma2(ny, splat2(-f.l_lo), fma2(ny, splat2(-f.l_hi), dy));
+    const float2 x = mul2(rx, splat2(f.unit)), y = mul2(ry, splat2(f.unit));
+    const float2 xm = mul2(rx, splat2(-f.unit)), ym = mul2(ry, splat2(-f.unit));
+    const float2 xx = mul2(x, x);
+    const float2 r = fma2(y, y, xx), a = fma2(y, ym, xx);
+    near0 = r.x < f.near2_unit;
+    near1 = r.y < f.near2_unit;
+    const float2 b4 = mul2(splat2(4.0f), mul2(x, y));
+    const float2 r2 = mul2(r, r), nn = mul2(r2, mul2(r2, splat2(-1.0f)));  // -|w|^2, w = z^4
+    const float2 wr = fma2(mul2(b4, b4), splat2(-0.5f), r2), wi = mul2(a, b4);
+    const float2 tr = add2(wr, wr);
+    const float2 p2 = fma2(tr, splat2(kP3), splat2(kP2));
+    const float2 p1 = fma2(tr, p2, fma2(nn, splat2(kP3), splat2(kP1)));
+    const float2 pr = fma2(wr, p1, fma2(nn, p2, splat2(kP0)));
+    const float2 pi = mul2(wi, p1), pim = mul2(pi, splat2(-1.0f));
+    const float2 q1 = add2(tr, splat2(kQ1));
+    const float2 qr = fma2(wr, q1, add2(nn, splat2(kQ0))), qi = mul2(wi, q1);
+    const float2 dr = fma2(x, qr, mul2(ym, qi)), di = fma2(x, qi, mul2(y, qr));  // z Q
+    const float2 den = fma2(dr, dr, mul2(di, di));
+    const float2 inv = make_float2(rcp_approx_f32(den.x), rcp_approx_f32(den.y));
+    const float2 ku2 = fma2(fma2(pr, di, mul2(pim, dr)), inv, mul2(ym, splat2(0.5f)));
+    const float2 kv2 = fma2(fma2(pr, dr, mul2(pi, di)), inv, mul2(xm, splat2(0.5f)));
+    ku = make_float2(near0 ? 0.0f : ku2.x, near1 ? 0.0f : ku2.y);
+    kv = make_float2(near0 ? 0.0f : kv2.x, near1 ? 0.0f : kv2.y);
+}
+
 // The plane's kernel values in FP32: K = (dy, dx) / (r^2 + eps^2) from the double-float
 // displacement. Exactly odd under exchanging target and source, as periodic_values32. The plane
 // has no near field.
@@ -218,13 +273,19 @@ __device__ __forceinline__ void plane_values32(const F32Geometry &f, const float
 // true for a near pair (terms 0, listed for the FP64 pass); kNear: the kernel has a near field.
 struct Periodic32 {
     static constexpr bool kNear = true;
+    static constexpr bool kPacked = false;
     __device__ __forceinline__ static bool values(const F32Geometry &f, const float4 t,
                                                   const float4 s, float &ku, float &kv) {
         return periodic_values32(f, t, s, ku, kv);
     }
 };
+// From six images up: whole tiles off the diagonal take zeta_values32_x2, the others Periodic32.
+struct Zeta32 : Periodic32 {
+    static constexpr bool kPacked = true;
+};
 struct Plane32 {
     static constexpr bool kNear = false;
+    static constexpr bool kPacked = false;
     __device__ __forceinline__ static bool values(const F32Geometry &f, const float4 t,
                                                   const float4 s, float &ku, float &kv) {
         plane_values32(f, t, s, ku, kv);

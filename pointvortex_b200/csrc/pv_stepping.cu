@@ -188,13 +188,17 @@ __device__ __forceinline__ void finish_target(const StageArgs &a, size_t i, doub
 // (at most f32::kNearSlots), each computes its entries' FP64 terms (the plain kernels' pair
 // functions) and their rank in (source, image) order, and the target's first thread adds them in
 // that order, so the sum does not depend on the order of the listing. A target with more
-// entries than slots is evaluated whole in FP64 instead (the threads striding over the sources,
-// their sums added in thread order), replacing its partial rows. Every count is reset.
+// entries than slots is evaluated whole in FP64 instead (every thread of the block striding over the
+// sources, their sums added in a fixed tree), replacing its partial rows. One such target among
+// N = 12 000 makes the stage 469 us when only its own 16 threads share it, 41 us so. Every
+// count is reset.
 // Returns, for the calling first thread (group 0) of target `lane`, the near sum (nu, nv) and
 // whether it replaces the rows.
 struct NearScratch {
     unsigned key[16][f32::kNearSlots];
     double tu[16][f32::kNearSlots], tv[16][f32::kNearSlots];
+    int over[16];             // targets evaluated whole
+    double warp_u[8], warp_v[8];
 };
 
 __device__ __forceinline__ bool fused_near(const NearPass &np, size_t i, bool valid, int lane,
@@ -204,31 +208,54 @@ __device__ __forceinline__ bool fused_near(const NearPass &np, size_t i, bool va
     // every thread of the target reads its count (the first one resets it after the barrier
     // below, once all have read it)
     const unsigned count = valid ? np.lists.count[gi] : 0u;
-    bool whole = false;
+    const bool whole = count > static_cast<unsigned>(f32::kNearSlots);
     nu = nv = 0.0;
     const double tx = valid && count ? np.x[gi] : 0.0, ty = valid && count ? np.y[gi] : 0.0;
-    if (count > static_cast<unsigned>(f32::kNearSlots)) {
-        // overflow: the whole target in FP64
-        double su = 0.0, sv = 0.0;
-        for (size_t j = group; j < np.n; j += groups) {
-            if (np.g.geometry == GEO_PERIODIC)
-                PeriodicPair::pair<true>(np.g, tx, ty, np.x[j], np.y[j], np.gs[j], j == gi, su,
-                                         sv);
-            else
-                DiskPair::pair<true>(np.g, tx, ty, np.x[j], np.y[j], np.gs[j], j == gi, su, sv);
-        }
-        sc.tu[lane][group] = su;
-        sc.tv[lane][group] = sv;
-        whole = true;
-    } else if (count) {
+    if (group == 0)
+        sc.over[lane] = whole ? 1 : 0;
+    if (!whole && count) {
         for (int e = group; e < static_cast<int>(count); e += groups) {
             const unsigned v = np.lists.slot[gi * f32::kNearSlots + e];
             sc.key[lane][e] = (v & ~f32::kNearImage) * 2u + (v >> 31);
         }
     }
-    __syncthreads();
+    const int any_over = __syncthreads_or(whole);
     if (group == 0 && count)
         np.lists.count[gi] = 0u;
+    if (any_over) {
+        const size_t first = gi - static_cast<size_t>(lane);  // the block's first target
+        for (int l = 0; l < 16; ++l) {
+            if (!sc.over[l])  // the same answer in every thread
+                continue;
+            const size_t t = first + l;
+            const double px = np.x[t], py = np.y[t];
+            double su = 0.0, sv = 0.0;
+            for (size_t j = threadIdx.x; j < np.n; j += blockDim.x) {
+                if (np.g.geometry == GEO_PERIODIC)
+                    periodic_pair<true>(np.g, px, py, np.x[j], np.y[j], np.gs[j], j == t, su, sv);
+                else
+                    DiskPair::pair<true>(np.g, px, py, np.x[j], np.y[j], np.gs[j], j == t, su, sv);
+            }
+            for (int off = 16; off > 0; off >>= 1) {
+                su += __shfl_down_sync(0xffffffffu, su, off);
+                sv += __shfl_down_sync(0xffffffffu, sv, off);
+            }
+            if ((threadIdx.x & 31) == 0) {
+                sc.warp_u[threadIdx.x >> 5] = su;
+                sc.warp_v[threadIdx.x >> 5] = sv;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int w = 1; w < 8; ++w) {
+                    su += sc.warp_u[w];
+                    sv += sc.warp_v[w];
+                }
+                sc.tu[l][0] = su;
+                sc.tv[l][0] = sv;
+            }
+            __syncthreads();
+        }
+    }
     if (!whole && count) {
         for (int e = group; e < static_cast<int>(count); e += groups) {
             const unsigned key = sc.key[lane][e];
@@ -240,7 +267,7 @@ __device__ __forceinline__ bool fused_near(const NearPass &np, size_t i, bool va
             if (key & 1u)
                 DiskPair::image(np.g, tx, ty, np.x[j], np.y[j], np.gs[j], du, dv);
             else if (np.g.geometry == GEO_PERIODIC)
-                PeriodicPair::pair<false>(np.g, tx, ty, np.x[j], np.y[j], np.gs[j], false, du, dv);
+                periodic_pair<false>(np.g, tx, ty, np.x[j], np.y[j], np.gs[j], false, du, dv);
             else
                 DiskPair::direct(tx, ty, np.x[j], np.y[j], np.gs[j], du, dv);
             sc.tu[lane][rank] = du;
@@ -249,7 +276,7 @@ __device__ __forceinline__ bool fused_near(const NearPass &np, size_t i, bool va
     }
     __syncthreads();
     if (group == 0 && count) {
-        const int terms = whole ? groups : static_cast<int>(count);
+        const int terms = whole ? 1 : static_cast<int>(count);
         for (int r = 0; r < terms; ++r) {
             nu += sc.tu[lane][r];
             nv += sc.tv[lane][r];

@@ -182,6 +182,7 @@ __global__ void __launch_bounds__(kThreads)
     extern __shared__ double2 reaction_smem[];
     __shared__ float4 src_f[kThreads];
     __shared__ float src_g[kThreads];
+    __shared__ sym::SourceBuffer32 packed_smem[V::kPacked ? kThreads / 32 : 1];
     pdl_enter();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double2 *reaction = reaction_smem + warp * a * 32;
@@ -277,12 +278,25 @@ __global__ void __launch_bounds__(kThreads)
                     const size_t sj = j0 + lane;
                     const int s_count =
                         j0 < n ? static_cast<int>(min(static_cast<size_t>(32), n - j0)) : 0;
+                    const float4 s = sym::split32(sj < n ? x[sj] : 0.0, sj < n ? y[sj] : 0.0);
+                    const float sg = sj < n ? static_cast<float>(gs[sj]) : 0.0f;
+                    const sym::NearTile nt{near, ti, j0};
+                    if constexpr (V::kPacked) {
+                        if (!(diagonal && jb == ib) &&
+                            __all_sync(0xffffffffu, t_ok && s_count == 32)) {
+                            sym::SourceBuffer32 &packed = packed_smem[warp];
+                            packed.fill(s, sg);
+                            double2 r = reaction[jb * 32 + lane];
+                            sym::react_tile_zeta32(f, t, tg, packed, ud, vd, r.x, r.y, nt);
+                            reaction[jb * 32 + lane] = r;
+                            continue;
+                        }
+                    }
                     __syncwarp();  // the previous tile's reads of the buffer are done
-                    sf[lane] = sym::split32(sj < n ? x[sj] : 0.0, sj < n ? y[sj] : 0.0);
-                    sgf[lane] = sj < n ? static_cast<float>(gs[sj]) : 0.0f;
+                    sf[lane] = s;
+                    sgf[lane] = sg;
                     __syncwarp();
                     float u = 0.0f, v = 0.0f;
-                    const sym::NearTile nt{near, ti, j0};
                     if (diagonal && jb == ib) {
                         sym::one_sided_tile32<V>(f, t, t_ok, sf, sgf, s_count, true, u, v, nt);
                     } else {
@@ -342,7 +356,8 @@ enum SymKernel : int {
     SYM_DISK = 13,        // the disk with one, two and four targets per lane
     SYM_DISK_T2 = 14,
     SYM_DISK_T4 = 15,
-    SYM_KERNELS = 16
+    SYM_ZETA32 = 16,      // the FP32C box from six images up
+    SYM_KERNELS = 17
 };
 
 int kernel_of(const SymmetricPlan &p) {
@@ -354,7 +369,7 @@ int kernel_of(const SymmetricPlan &p) {
     if (p.geometry == GEO_DISK)
         return p.targets == 4 ? SYM_DISK_T4 : (p.targets == 2 ? SYM_DISK_T2 : SYM_DISK);
     if (fp32c)
-        return SYM_PERIODIC32;
+        return p.zeta ? SYM_ZETA32 : SYM_PERIODIC32;
     if (p.targets == 2)
         return p.zeta ? SYM_ZETA_T2 : SYM_PERIODIC_T2;
     if (p.zeta)
@@ -382,6 +397,9 @@ int resident_ctas(int a, int kernel) {
         const size_t smem = static_cast<size_t>(kThreads / 32) * a * 32 * sizeof(double2);
         int blocks = 1;
         switch (kernel) {
+        case SYM_ZETA32:
+            blocks = occupancy(symmetric32_kernel<f32::Zeta32, 1>, smem);
+            break;
         case SYM_PERIODIC32:
             blocks = occupancy(symmetric32_kernel<f32::Periodic32, 1>, smem);
             break;
@@ -522,7 +540,11 @@ SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const Geomet
               : (precision == PV_PRECISION_FP64 && tuned_targets == 2 ? 2 : 1);
     p.min_ctas = tuned_ctas;
     const size_t np = (n + 255) & ~static_cast<size_t>(255);
-    for (int a = targets; a <= 16; a *= 2) {
+    // The FP32C box's packed tiles take half the time of the other form's, so from 8192 (32 768)
+    // blocks of two (four) sub-blocks balance as well and halve (quarter) the rows to reduce
+    const int first = precision == PV_PRECISION_FP32C && g.zeta ? (n >= 32768 ? 4 : n >= 8192 ? 2 : 1)
+                                                                : targets;
+    for (int a = first; a <= 16; a *= 2) {
         const size_t blocks = (n + 32 * static_cast<size_t>(a) - 1) / (32 * static_cast<size_t>(a));
         if (blocks > 0xffffu)
             continue;
@@ -563,6 +585,9 @@ cudaError_t launch_symmetric(const double *x, const double *y, const double *gs,
     const size_t smem = static_cast<size_t>(kThreads / 32) * p.a * 32 * sizeof(double2);
     const dim3 grid(static_cast<unsigned>(p.grid)), block(kThreads);
     switch (kernel_of(p)) {
+    case SYM_ZETA32:
+        return launch_pdl(symmetric32_kernel<f32::Zeta32, 1>, grid, block, smem, stream, x, y, gs, n,
+                          p.a, items, p.items, counter, rows, stride, g, near);
     case SYM_PERIODIC32:
         return launch_pdl(symmetric32_kernel<f32::Periodic32, 1>, grid, block, smem, stream, x, y,
                           gs, n, p.a, items, p.items, counter, rows, stride, g, near);

@@ -357,6 +357,78 @@ __device__ __forceinline__ void react_tile32(const f32::F32Geometry &f, const fl
         react_tile32_t<V, false>(f, t, tg, t_ok, sf, sg, s_count, u, v, ru, rv, nt);
 }
 
+// The sources of a whole tile packed for zeta_values32_x2: entry j holds source j & 31 and, in the
+// other f32x2 lane, source (j + 16) & 31, so that step k of lane l (k < 16) reads entry l + k and
+// meets both. Coordinates negated.
+struct SourceBuffer32 {
+    float4 hi[48];  // (-xh_j, -xh_j+16, -yh_j, -yh_j+16)
+    float4 lo[48];
+    float4 g[48];   // (-g_j, -g_j+16, g_j, g_j+16)
+    __device__ __forceinline__ void fill(const float4 s, float sg) {
+        const int lane = threadIdx.x & 31;
+        float4 o;
+        o.x = __shfl_xor_sync(0xffffffffu, s.x, 16);
+        o.y = __shfl_xor_sync(0xffffffffu, s.y, 16);
+        o.z = __shfl_xor_sync(0xffffffffu, s.z, 16);
+        o.w = __shfl_xor_sync(0xffffffffu, s.w, 16);
+        const float og = __shfl_xor_sync(0xffffffffu, sg, 16);
+        const float4 h = make_float4(-s.x, -o.x, -s.y, -o.y), l = make_float4(-s.z, -o.z, -s.w, -o.w);
+        __syncwarp();  // the previous tile's reads are done
+        hi[lane] = h;
+        lo[lane] = l;
+        const float4 gg = make_float4(-sg, -og, sg, og);
+        g[lane] = gg;
+        if (lane < 16) {
+            hi[lane + 32] = h;
+            lo[lane + 32] = l;
+            g[lane + 32] = gg;
+        }
+        __syncwarp();
+    }
+};
+
+// A whole tile of 32 targets and the buffer's 32 sources in 16 steps of two pairs a lane. Each FP32
+// sum covers 16 terms; a target's two (one a lane of the pair) and a source's two are added in FP64.
+__device__ __forceinline__ void react_tile_zeta32(const f32::F32Geometry &f, const float4 t,
+                                                  float tg, const SourceBuffer32 &b, double &ud,
+                                                  double &vd, double &rud, double &rvd,
+                                                  const NearTile &nt) {
+    const int lane = threadIdx.x & 31, next = (lane + 1) & 31;
+    const float2 thx = f32::splat2(t.x), thy = f32::splat2(t.y), tlx = f32::splat2(t.z),
+                 tly = f32::splat2(t.w), tg2 = f32::splat2(tg), tgm2 = f32::splat2(-tg);
+    float2 u = f32::splat2(0.0f), v = u, ru = u, rv = u;
+#pragma unroll 2
+    for (int k = 0; k < 16; ++k) {
+        const float4 h = b.hi[lane + k], l = b.lo[lane + k];
+        const float4 g = b.g[lane + k];
+        float2 ku, kv;
+        bool near0, near1;
+        f32::zeta_values32_x2(f, thx, thy, tlx, tly, make_float2(h.x, h.y), make_float2(h.z, h.w),
+                              make_float2(l.x, l.y), make_float2(l.z, l.w), ku, kv, near0, near1);
+        if (near0 || near1) {
+            if (near0)
+                list_near_pair<f32::Periodic32>(nt, (lane + k) & 31, true);
+            if (near1)
+                list_near_pair<f32::Periodic32>(nt, (lane + k + 16) & 31, true);
+        }
+        u = f32::fma2(make_float2(g.x, g.y), ku, u);
+        v = f32::fma2(make_float2(g.z, g.w), kv, v);
+        ru = f32::fma2(tg2, ku, ru);
+        rv = f32::fma2(tgm2, kv, rv);
+        ru.x = __shfl_sync(0xffffffffu, ru.x, next);
+        ru.y = __shfl_sync(0xffffffffu, ru.y, next);
+        rv.x = __shfl_sync(0xffffffffu, rv.x, next);
+        rv.y = __shfl_sync(0xffffffffu, rv.y, next);
+    }
+    ud += static_cast<double>(u.x) + static_cast<double>(u.y);
+    vd += static_cast<double>(v.x) + static_cast<double>(v.y);
+    // after 16 rotations lane l holds source l's second sum and source l + 16's first
+    rud += static_cast<double>(ru.y) +
+           static_cast<double>(__shfl_xor_sync(0xffffffffu, ru.x, 16));
+    rvd += static_cast<double>(rv.y) +
+           static_cast<double>(__shfl_xor_sync(0xffffffffu, rv.x, 16));
+}
+
 // T targets per lane against the 32 sources of the buffer, every target and source present: each
 // step serves T pairs per lane, and the reactions' two shuffles are shared by them. Only for pair
 // kernels without a near field (the plane): a near verdict is not acted on here. A reaction
