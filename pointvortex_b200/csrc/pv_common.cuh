@@ -41,7 +41,11 @@ struct DeviceControl {
     double dt;                 // DOPRI5: step size of the current attempt
     double absolute_tolerance, relative_tolerance, minimum_time_step, maximum_time_step;
     double result[4];          // accepted dt, suggested dt, normalised error, rejected
-    double pad[18];
+    unsigned long long err_bits2; // cooperative DOPRI5 steps: err_bits of every second attempt
+    int attempts;              // cooperative DOPRI5 steps: attempts begun
+    int pad1;
+    double pad[15];
+    unsigned long long arrivals; // the cooperative steps' grid barrier
 };
 static_assert(sizeof(DeviceControl) == 256, "control block is one 256-byte line");
 

@@ -39,6 +39,9 @@ constexpr double kB5[7] = {35.0 / 384.0,     0.0,         500.0 / 1113.0, 125.0 
 constexpr double kB4[7] = {5179.0 / 57600.0, 0.0,          7571.0 / 16695.0,   393.0 / 640.0,
                            -92097.0 / 339200.0, 187.0 / 2100.0, 1.0 / 40.0};
 
+// Stage rows of the classical Runge–Kutta method, src/timestep.cpp:38-50.
+constexpr double kRk4[3][3] = {{0.5}, {0.0, 0.5}, {0.0, 0.0, 1.0}};
+
 // A growable device allocation.
 struct DeviceArray {
     double *p = nullptr;
@@ -96,7 +99,6 @@ struct pv_context {
     cudaGraphExec_t attempt_graph = nullptr; // one DOPRI5 attempt with a valid FSAL derivative
     SymmetricPlan sym{};             // one evaluation per unordered pair (when planned)
     DeviceArray sym_items, sym_counter;
-    DeviceArray rk4_barrier;         // arrival counter of the cooperative RK4 steps' grid barrier
     int sym_items_blocks = 0;        // the block count the item table was built for
     DeviceArray inv_scratch, inv_out;
     DeviceArray cand;                // dipole candidates (3 doubles-worth each)
@@ -156,7 +158,7 @@ struct pv_context {
         for (DeviceArray *a : {&x, &y, &gamma, &gs, &p0x, &p0y, &p1x, &p1y, &pu, &pv, &inv_scratch,
                                &inv_out, &cand, &ex, &ey, &eg, &egs, &eu, &ev, &epu, &epv,
                                &removed_index, &fmt_stage, &fmt_len, &fmt_block, &fmt_out,
-                               &sym_items, &sym_counter, &rk4_barrier, &near_count, &near_slot})
+                               &sym_items, &sym_counter, &near_count, &near_slot})
             a->release();
         for (int s = 0; s < 7; ++s) {
             kx[s].release();
@@ -1015,7 +1017,6 @@ namespace {
 // previous stage's position, writing the next position into the ping-pong buffers; stage 3
 // writes the combined state.
 StageArgs rk4_stage(pv_context *c, double dt, int s) {
-    static const double rows[3][3] = {{0.5}, {0.0, 0.5}, {0.0, 0.0, 1.0}};
     double *pos_x[2] = {c->p0x.p, c->p1x.p};
     double *pos_y[2] = {c->p0y.p, c->p1y.p};
     StageArgs a = stage_base(c);
@@ -1029,39 +1030,51 @@ StageArgs rk4_stage(pv_context *c, double dt, int s) {
         a.mode = STAGE_POSITION;
         a.ncoef = s + 1;
         for (int j = 0; j <= s; ++j)
-            a.coef[j] = rows[s][j];
+            a.coef[j] = kRk4[s][j];
     } else {
         a.mode = STAGE_RK4_COMBINE;
     }
     return a;
 }
 
-// Whole RK4 steps in one cooperative launch: FP64, the ordered kernel's plan (no symmetric
-// rows), a small enough population, and no per-launch profiling.
-bool rk4_steps_apply(const pv_context *c) {
+// Whole steps in one cooperative launch: FP64, the ordered kernel's plan (no symmetric rows), a
+// small enough population, and no per-launch profiling.
+bool small_steps_apply(const pv_context *c) {
     return !c->profiling && c->params.precision == PV_PRECISION_FP64 && !c->sym.enabled() &&
-           rk4_steps_eligible(c->n, c->plan.num_chunks);
+           small_steps_eligible(c->n, c->plan.num_chunks, c->sm_count);
 }
 
-pv_status enqueue_rk4_steps(pv_context *c, double dt, uint64_t steps) {
-    Rk4Steps p{};
-    for (int s = 0; s < 4; ++s)
-        p.stage[s] = rk4_stage(c, dt, s);
+pv_status enqueue_small_steps(pv_context *c, SmallSteps &p) {
     p.x = c->x.p;
     p.y = c->y.p;
+    p.gamma = c->gamma.p;
     p.gs = c->gs.p;
     p.n = c->n;
     p.chunk = c->plan.chunk;
     p.num_chunks = c->plan.num_chunks;
-    p.steps = steps;
+    p.px[0] = c->p0x.p;
+    p.px[1] = c->p1x.p;
+    p.py[0] = c->p0y.p;
+    p.py[1] = c->p1y.p;
+    p.k0x = c->kx[0].p;
+    p.k0y = c->ky[0].p;
+    p.ctl = c->ctl;
     p.spin_limit = c->spin_limit;
-    PV_CUDA(c, c->rk4_barrier.ensure(1));
-    PV_CUDA(c, cudaMemsetAsync(c->rk4_barrier.p, 0, sizeof(unsigned long long), c->stream));
-    p.barrier = reinterpret_cast<unsigned long long *>(c->rk4_barrier.p);
+    p.g = c->gc;
     PV_CUDA(c, counted(c, PV_KERNEL_VELOCITY, 1,
-                       [&] { return launch_rk4_steps(p, c->sm_count, c->stream); }));
-    c->evaluations += 4 * steps;
+                       [&] { return launch_small_steps(p, c->sm_count, c->stream); }));
     return PV_OK;
+}
+
+pv_status enqueue_rk4_steps(pv_context *c, double dt, uint64_t steps) {
+    SmallSteps p{};
+    for (int s = 0; s < 3; ++s)
+        for (int j = 0; j <= s; ++j)
+            p.rows[s + 1][j] = kRk4[s][j];
+    p.steps = steps;
+    p.dt = dt;
+    c->evaluations += 4 * steps;
+    return enqueue_small_steps(c, p);
 }
 
 pv_status enqueue_rk4(pv_context *c, double dt) {
@@ -1099,7 +1112,7 @@ pv_status pv_rk4_step(pv_context *ctx, double dt) {
     DeviceGuard guard(ctx->device);
     if ((st = reset_control(ctx)) != PV_OK)
         return st;
-    if ((st = rk4_steps_apply(ctx) ? enqueue_rk4_steps(ctx, dt, 1) : enqueue_rk4(ctx, dt)) != PV_OK)
+    if ((st = small_steps_apply(ctx) ? enqueue_rk4_steps(ctx, dt, 1) : enqueue_rk4(ctx, dt)) != PV_OK)
         return st;
     if ((st = read_control(ctx)) != PV_OK)
         return st;
@@ -1121,7 +1134,7 @@ pv_status pv_rk4_advance(pv_context *ctx, double dt, uint64_t steps) {
     DeviceGuard guard(ctx->device);
     if ((st = reset_control(ctx)) != PV_OK)
         return st;
-    if (rk4_steps_apply(ctx)) {
+    if (small_steps_apply(ctx)) {
         if ((st = enqueue_rk4_steps(ctx, dt, steps)) != PV_OK)
             return st;
     } else if (ctx->profiling || steps < 4) {
@@ -1175,6 +1188,18 @@ pv_status pv_rk4_advance(pv_context *ctx, double dt, uint64_t steps) {
 }
 
 namespace {
+// The dipole scan of the state an attempt accepted (the kernel returns at once after a rejection).
+pv_status enqueue_prescan(pv_context *ctx) {
+    auto *dev = reinterpret_cast<DipoleCandidateDev *>(ctx->cand.p);
+    auto *dev_count = reinterpret_cast<unsigned long long *>(&ctx->ctl->dipole_count);
+    PV_CUDA(ctx, counted(ctx, PV_KERNEL_DIPOLE, 1, [&] {
+                return launch_dipole_scan(ctx->x.p, ctx->y.p, ctx->gamma.p, ctx->n, ctx->gc,
+                                          ctx->dipole.distance, dev, ctx->cand.cap / 3, dev_count,
+                                          ctx->stream, ctx->ctl);
+            }));
+    return PV_OK;
+}
+
 // One DOPRI5 attempt (src/timestep.cpp:62-120) on the context stream: k0 when it is not cached,
 // stages 1..6 with their positions, the error norm and step control of the last stage, and the
 // accept kernel. Everything it needs from the host is in the control block.
@@ -1223,16 +1248,8 @@ pv_status enqueue_dopri_attempt(pv_context *ctx, bool need_k0) {
                 return launch_accept(ctx->x.p, ctx->y.p, px, py, ctx->kx[0].p, ctx->ky[0].p,
                                      ctx->kx[6].p, ctx->ky[6].p, ctx->n, 1, ctx->ctl, ctx->stream);
             }));
-    if (ctx->dipole_configured && ctx->dipole.removal) {
-        // the dipole scan of the accepted state (the kernel returns at once after a rejection)
-        auto *dev = reinterpret_cast<DipoleCandidateDev *>(ctx->cand.p);
-        auto *dev_count = reinterpret_cast<unsigned long long *>(&ctx->ctl->dipole_count);
-        PV_CUDA(ctx, counted(ctx, PV_KERNEL_DIPOLE, 1, [&] {
-                    return launch_dipole_scan(ctx->x.p, ctx->y.p, ctx->gamma.p, ctx->n, ctx->gc,
-                                              ctx->dipole.distance, dev, ctx->cand.cap / 3,
-                                              dev_count, ctx->stream, ctx->ctl);
-                }));
-    }
+    if (ctx->dipole_configured && ctx->dipole.removal)
+        return enqueue_prescan(ctx);
     return PV_OK;
 }
 } // namespace
@@ -1273,6 +1290,39 @@ pv_status pv_dopri5_step(pv_context *ctx, double dt, double absolute_tolerance,
     if (prescan)
         PV_CUDA(ctx, ctx->cand.ensure(3 * 64));
     bool need_k0 = !ctx->fsal_valid;
+    const auto accept = [&] {
+        ctx->fsal_valid = true;
+        ctx->prescan_valid = prescan;
+        ctx->prescan_count = ctx->ctl_host->dipole_count;
+        result->accepted_time_step = ctx->ctl_host->result[0];
+        result->suggested_time_step = ctx->ctl_host->result[1];
+        result->normalized_error = ctx->ctl_host->result[2];
+        result->rejected_steps = static_cast<unsigned>(ctx->ctl_host->result[3]);
+    };
+    if (small_steps_apply(ctx)) {
+        // every attempt of the step in one launch, then the dipole scan of the accepted state
+        SmallSteps p{};
+        p.dopri = 1;
+        p.need_k0 = need_k0 ? 1 : 0;
+        for (int s = 0; s < 7; ++s) {
+            for (int j = 0; j < 7; ++j)
+                p.rows[s][j] = kDopri[s][j];
+            p.w[s] = kB5[s] - kB4[s];
+        }
+        if ((st = enqueue_small_steps(ctx, p)) != PV_OK)
+            return st;
+        if (prescan && (st = enqueue_prescan(ctx)) != PV_OK)
+            return st;
+        if ((st = read_control(ctx)) != PV_OK)
+            return st;
+        ctx->evaluations += (need_k0 ? 1u : 0u) + 6u * static_cast<uint64_t>(ctx->ctl_host->attempts);
+        if (ctx->ctl_host->status != 0) {
+            ctx->fsal_valid = false;
+            return status_error(ctx, ctx->ctl_host->status);
+        }
+        accept();
+        return PV_OK;
+    }
     for (int attempt = 0; attempt < 40; ++attempt) {
         if (need_k0) {
             if ((st = enqueue_dopri_attempt(ctx, need_k0)) != PV_OK)
@@ -1339,13 +1389,7 @@ pv_status pv_dopri5_step(pv_context *ctx, double dt, double absolute_tolerance,
             return status_error(ctx, ctx->ctl_host->status);
         }
         if (ctx->ctl_host->accepted) {
-            ctx->fsal_valid = true;
-            ctx->prescan_valid = prescan;
-            ctx->prescan_count = ctx->ctl_host->dipole_count;
-            result->accepted_time_step = ctx->ctl_host->result[0];
-            result->suggested_time_step = ctx->ctl_host->result[1];
-            result->normalized_error = ctx->ctl_host->result[2];
-            result->rejected_steps = static_cast<unsigned>(ctx->ctl_host->result[3]);
+            accept();
             return PV_OK;
         }
     }

@@ -178,26 +178,33 @@ struct StageArgs {
 
 cudaError_t launch_stage(const StageArgs &a, cudaStream_t stream, int sm_count);
 
-// Polls a grid barrier of the cooperative RK4 steps waits before it gives up (ST_TIMEOUT).
+// Polls a grid barrier of the cooperative steps waits before it gives up (ST_TIMEOUT).
 constexpr uint32_t kGridSpinLimit = 1u << 24;
 
-// RK4 steps of a small FP64 population in one cooperative launch (pv_stepping.cu): the four
-// stages as enqueue_rk4 sets them up (stage[3].xt/yt: the combined state), bit for bit the same
-// results as launching them. barrier: the grid barrier's arrival counter, zero at every
-// launch. Eligible up to kRk4StepsMaxN vortices with fewer than 32 chunks.
-struct Rk4Steps {
-    StageArgs stage[4];
-    double *x, *y;          // the state, updated after every step
-    const double *gs;       // scaled circulations
+// Whole steps of a small FP64 population in one cooperative launch (pv_stepping.cu): `steps` RK4 steps,
+// or one DOPRI5 step with its rejected attempts; bit for bit the same results as the launch
+// sequence. The control block is zero but for the step's inputs at every launch (the grid barrier
+// counts in it). Eligible up to kSmallStepsMaxN vortices with fewer than 32 chunks.
+struct SmallSteps {
+    int dopri;              // one DOPRI5 step (dt and tolerances in ctl) instead of RK4 steps
+    int need_k0;            // DOPRI5: evaluate the derivative at the state first
+    double *x, *y;          // the state
+    const double *gamma, *gs;  // circulations, raw and scaled
     size_t n;
     int chunk, num_chunks;  // the ordered kernel's source chunks
+    double *px[2], *py[2];  // exchanged positions
+    double *k0x, *k0y;      // DOPRI5: the cached derivative
+    double rows[7][7];      // the tableau: rows[s + 1] gives the position of stage s + 1
+    double w[7];            // DOPRI5: b5 - b4
     uint64_t steps;
-    unsigned long long *barrier;
+    double dt;
+    DeviceControl *ctl;
     uint32_t spin_limit = kGridSpinLimit;  // polls of a grid-barrier wait (pv_set_wait_limits)
+    GeometryConsts g;
 };
-constexpr size_t kRk4StepsMaxN = 2048;
-bool rk4_steps_eligible(size_t n, int num_chunks);
-cudaError_t launch_rk4_steps(const Rk4Steps &p, int sm_count, cudaStream_t stream);
+constexpr size_t kSmallStepsMaxN = 2048;
+bool small_steps_eligible(size_t n, int num_chunks, int sm_count);
+cudaError_t launch_small_steps(const SmallSteps &p, int sm_count, cudaStream_t stream);
 
 // Accept kernel: state <- xt (and, for DOPRI5, k0 <- k6 when the attempt was accepted).
 cudaError_t launch_accept(double *x, double *y, const double *xt, const double *yt, double *k0x,

@@ -144,8 +144,8 @@ __global__ void __launch_bounds__(kHT)
                     term = log(r2);
                 } else if (ZETA) {
                     bool coincident;
-                    term = box_energy(gc, ZetaPair::reduce(gc, xi - xj, gc.lx, gc.inv_lx),
-                                      ZetaPair::reduce(gc, yi - yj, gc.ly, gc.inv_ly), coincident);
+                    term = box_energy(gc, ZetaPair::reduce_any(gc, xi - xj, gc.lx, gc.inv_lx),
+                                      ZetaPair::reduce_any(gc, yi - yj, gc.ly, gc.inv_ly), coincident);
                     if (coincident)
                         set_status(status, ST_COINCIDENT);
                 } else if (GEO == GEO_PERIODIC) {

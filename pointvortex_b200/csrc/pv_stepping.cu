@@ -31,36 +31,76 @@ __device__ __forceinline__ double clamp_ref(double v, double lo, double hi) {
     return v < lo ? lo : (hi < v ? hi : v);
 }
 
-// Validation of a new position, src/vortex.h:7-14 and src/compute.cpp:41-48.
-__device__ __forceinline__ void validate_position(const StageArgs &a, double x, double y) {
+// Verdict on a new position (0: valid), src/vortex.h:7-14 and src/compute.cpp:41-48.
+__device__ __forceinline__ int position_error(const GeometryConsts &g, double x, double y) {
     if (!isfinite(x) || !isfinite(y))
-        set_status(&a.ctl->status, ST_NONFINITE_POSITION);
-    else if (a.g.geometry == GEO_DISK &&
-             __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)) >= a.g.radius2)
-        set_status(&a.ctl->status, ST_OUTSIDE_DISK);
+        return ST_NONFINITE_POSITION;
+    if (g.geometry == GEO_DISK && __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)) >= g.radius2)
+        return ST_OUTSIDE_DISK;
+    return 0;
 }
 
-// DOPRI5 step-size control, src/timestep.cpp:95-118, run by one thread.
+__device__ __forceinline__ void validate_position(const StageArgs &a, double x, double y) {
+    const int e = position_error(a.g, x, y);
+    if (e)
+        set_status(&a.ctl->status, e);
+}
+
+// src/timestep.cpp:52-57: x0 + dt * (k1 + 2 k2 + 2 k3 + k4) / 6
+__device__ __forceinline__ double rk4_point(double x0, double dt, double k1, double k2, double k3,
+                                            double k4) {
+    const double s = __dadd_rn(
+        __dadd_rn(__dadd_rn(k1, __dmul_rn(2.0, k2)), __dmul_rn(2.0, k3)), k4);
+    return __dadd_rn(x0, __ddiv_rn(__dmul_rn(dt, s), 6.0));
+}
+
+// The scale of an error component, src/timestep.cpp:84-87.
+__device__ __forceinline__ double error_scale(const DeviceControl *ctl, double x0, double x5) {
+    return __dadd_rn(ctl->absolute_tolerance,
+                     __dmul_rn(ctl->relative_tolerance, max_ref(fabs(x0), fabs(x5))));
+}
+
+// DOPRI5 step-size control, src/timestep.cpp:95-118. Returns ST_DOPRI_FAILED, or 0.
+__device__ __forceinline__ int dopri_decide(double error, double dt, double minimum,
+                                            double maximum, unsigned &rejected, int &accepted,
+                                            double &suggested, double &next_dt) {
+    const double factor = error == 0.0 ? 5.0 : clamp_ref(0.9 * pow(error, -0.2), 0.2, 5.0);
+    suggested = clamp_ref(__dmul_rn(dt, factor), minimum, maximum);
+    next_dt = dt;
+    accepted = error <= 1.0 ? 1 : 0;
+    if (accepted)
+        return 0;
+    if (dt <= minimum || ++rejected > 32u)
+        return ST_DOPRI_FAILED;
+    next_dt = max_ref(minimum, min_ref(suggested, __dmul_rn(dt, 0.9)));
+    return 0;
+}
+
+__device__ __forceinline__ void store_accepted(DeviceControl *ctl, double dt, double suggested,
+                                               double error, unsigned rejected) {
+    ctl->result[0] = dt;
+    ctl->result[1] = suggested;
+    ctl->result[2] = error;
+    ctl->result[3] = static_cast<double>(rejected);
+}
+
+// The control of an attempt made by launches, run by one thread.
 __device__ void dopri_control(DeviceControl *ctl) {
     const double error = __longlong_as_double(static_cast<long long>(ctl->err_bits));
     const double dt = ctl->dt;
-    const double factor = error == 0.0 ? 5.0 : clamp_ref(0.9 * pow(error, -0.2), 0.2, 5.0);
-    const double suggested =
-        clamp_ref(__dmul_rn(dt, factor), ctl->minimum_time_step, ctl->maximum_time_step);
     if (ctl->status == 0) {
-        if (error <= 1.0) {
-            ctl->accepted = 1;
-            ctl->result[0] = dt;
-            ctl->result[1] = suggested;
-            ctl->result[2] = error;
-            ctl->result[3] = static_cast<double>(ctl->rejected);
-        } else {
-            ctl->accepted = 0;
-            if (dt <= ctl->minimum_time_step || ++ctl->rejected > 32u)
-                set_status(&ctl->status, ST_DOPRI_FAILED);
-            else
-                ctl->dt = max_ref(ctl->minimum_time_step, min_ref(suggested, __dmul_rn(dt, 0.9)));
-        }
+        double suggested, next_dt;
+        unsigned rejected = ctl->rejected;
+        int accepted;
+        const int failed = dopri_decide(error, dt, ctl->minimum_time_step, ctl->maximum_time_step,
+                                        rejected, accepted, suggested, next_dt);
+        ctl->accepted = accepted;
+        ctl->rejected = rejected;
+        ctl->dt = next_dt;
+        if (accepted)
+            store_accepted(ctl, dt, suggested, error, rejected);
+        if (failed)
+            set_status(&ctl->status, failed);
     }
     ctl->err_bits = 0ull;
     ctl->blocks_done = 0u;
@@ -139,15 +179,8 @@ __device__ __forceinline__ void finish_target(const StageArgs &a, size_t i, doub
         a.yt[i] = ny;
         validate_position(a, nx, ny);
     } else if (MODE == STAGE_RK4_COMBINE) {
-        // src/timestep.cpp:52-57: x0 + dt * (k1 + 2 k2 + 2 k3 + k4) / 6
-        const double sx = __dadd_rn(__dadd_rn(__dadd_rn(p.kx[0], __dmul_rn(2.0, p.kx[1])),
-                                              __dmul_rn(2.0, p.kx[2])),
-                                    ku);
-        const double sy = __dadd_rn(__dadd_rn(__dadd_rn(p.ky[0], __dmul_rn(2.0, p.ky[1])),
-                                              __dmul_rn(2.0, p.ky[2])),
-                                    kv);
-        const double nx = __dadd_rn(p.x0, __ddiv_rn(__dmul_rn(dt, sx), 6.0));
-        const double ny = __dadd_rn(p.y0, __ddiv_rn(__dmul_rn(dt, sy), 6.0));
+        const double nx = rk4_point(p.x0, dt, p.kx[0], p.kx[1], p.kx[2], ku);
+        const double ny = rk4_point(p.y0, dt, p.ky[0], p.ky[1], p.ky[2], kv);
         a.xt[i] = nx;
         a.yt[i] = ny;
         if (!isfinite(nx) || !isfinite(ny))
@@ -167,12 +200,7 @@ __device__ __forceinline__ void finish_target(const StageArgs &a, size_t i, doub
             ye = __dadd_rn(ye, __dmul_rn(h, kyj));
         }
         const double x5 = p.xt, y5 = p.yt;
-        const double xs = __dadd_rn(a.ctl->absolute_tolerance,
-                                    __dmul_rn(a.ctl->relative_tolerance,
-                                              max_ref(fabs(p.x0), fabs(x5))));
-        const double ys = __dadd_rn(a.ctl->absolute_tolerance,
-                                    __dmul_rn(a.ctl->relative_tolerance,
-                                              max_ref(fabs(p.y0), fabs(y5))));
+        const double xs = error_scale(a.ctl, p.x0, x5), ys = error_scale(a.ctl, p.y0, y5);
         if (!isfinite(xe) || !isfinite(ye) || !isfinite(xs) || !isfinite(ys) || !(xs > 0.0) ||
             !(ys > 0.0)) {
             set_status(&a.ctl->status, ST_DOPRI_NONFINITE);
@@ -285,6 +313,26 @@ __device__ __forceinline__ bool fused_near(const NearPass &np, size_t i, bool va
     return whole;
 }
 
+// Fewer than kWideRows rows: four interleaved sums (rows 0, 4, 8, ...; 1, 5, ...), so that a chain of
+// dependent additions is a quarter of the rows long, and four rows are in flight. The cooperative
+// steps add their chunks in the same order.
+template <class Row>
+__device__ __forceinline__ void sum_chunks(int rows, Row &&row, double &ku, double &kv) {
+    double u[4] = {0.0, 0.0, 0.0, 0.0}, v[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int c = 0; c < rows; c += 4) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (c + q < rows) {
+                double ru, rv;
+                row(c + q, ru, rv);
+                u[q] += ru;
+                v[q] += rv;
+            }
+    }
+    ku = (u[0] + u[1]) + (u[2] + u[3]);
+    kv = (v[0] + v[1]) + (v[2] + v[3]);
+}
+
 // WIDE: many partial rows (the symmetric kernel's). A block then covers kWideTargets targets with
 // 256 / kWideTargets row groups: thread (group, t) sums rows group, group + groups, ...
 // (coalesced over the targets), and the threads of group 0 add the group sums in fixed order.
@@ -383,18 +431,17 @@ __global__ void __launch_bounds__(256) stage_kernel(const StageArgs a) {
              i += static_cast<size_t>(gridDim.x) * blockDim.x) {
             double ku, kv;
             if (a.reduce) {
-                ku = 0.0;
-                kv = 0.0;
-                for (int c = 0; c < a.num_chunks; ++c) {
+                const auto row = [&](int c, double &ru, double &rv) {
                     if (a.pr) {
                         const double2 r = a.pr[static_cast<size_t>(c) * a.stride + i];
-                        ku += r.x;
-                        kv += r.y;
+                        ru = r.x;
+                        rv = r.y;
                     } else {
-                        ku += a.pu[static_cast<size_t>(c) * a.stride + i];
-                        kv += a.pv[static_cast<size_t>(c) * a.stride + i];
+                        ru = a.pu[static_cast<size_t>(c) * a.stride + i];
+                        rv = a.pv[static_cast<size_t>(c) * a.stride + i];
                     }
-                }
+                };
+                sum_chunks(a.num_chunks, row, ku, kv);
             } else {
                 ku = a.kx[a.s][i];
                 kv = a.ky[a.s][i];
@@ -492,168 +539,400 @@ cudaError_t launch_stage(const StageArgs &a, cudaStream_t stream, int sm_count) 
 }
 
 // ---------------------------------------------------------------------------------------------
-// RK4 steps of a small population in one cooperative launch. Below N ~ 2000 a step's nine
-// launches take longer to schedule than to run, so one CTA per SM keeps the whole step loop: each
-// CTA owns a range of targets, and a grid barrier separates the four evaluations of a step.
+// Whole steps of a small FP64 population in one cooperative launch: RK4 steps, or one adaptive DOPRI5
+// step with its rejected attempts. Below N ~ 2000 a step's launches (9 for RK4, 13 an attempt) take
+// longer to schedule than to run, so one CTA per SM keeps the whole loop: each CTA owns a range of
+// targets, and a grid barrier separates the evaluations.
 //
-// The results are bit for bit those of the launch sequence (enqueue_rk4): a target's velocity is
-// summed chunk by chunk (the ordered kernel's chunks, sources in index order, pair<true> with the
-// self flag) and the chunk sums are added in chunk order from 0.0, as the stage kernel does with
-// fewer than kWideRows chunks; finish_target then runs unchanged. The previous step's combined
-// state (stage 3's output) is the next step's evaluation point and is copied into the state target
-// by target in the phase that reads it, so a step costs four barriers.
+// The results are bit for bit those of the launch sequence: a target's velocity is summed chunk by
+// chunk (the ordered kernel's chunks, sources in index order, pair<true> with the self flag), the
+// chunk sums are added as sum_chunks adds them, and the stage arithmetic is the stage kernel's.
+//
+// What bounds it is latency. One stage of N = 1024 in the plane: the barrier (arrival and poll, each a
+// round trip to L2), the load of all positions into shared memory, the chunk sums (up to 31 chunks,
+// so that 217 threads of an SM have one; their sources unrolled, so that the pairs' chains overlap)
+// and the finish, whose inputs -- the step's start and the earlier stage velocities -- stay in
+// shared memory: 0.9, 2.9, 1.5 and 2.4 thousand cycles for load, sums, finish and barrier. Measured
+// against the previous kernel (RK4, us a step: 128 threads' worth of chunks, positions and inputs
+// reloaded in the finish, a fenced atomic and a status read a barrier): plane N = 64 20 -> 14, 1024
+// 33 -> 17, 2047 47 -> 33; disk 2048 87 -> 52; box 1024 130 -> 31 (with ZetaPair). DOPRI5 against the
+// captured graph of launches (us a step, host included): disk 301 85 -> 57, plane 1024 81 -> 58, box
+// 1024 192 -> 83.
 
-// Grid barrier over the CTAs of a cooperative launch. The arrival counter starts at zero (the
-// host clears it before the launch) and only grows: the r-th barrier is open once it reaches
-// r * gridDim.x. One fence and one atomic per CTA, then polling with an acquire load.
+// Grid barrier over the CTAs of a cooperative launch. The arrival counter starts at zero (the control
+// block is reset before the launch) and only grows: the low 40 bits count arrivals, the r-th barrier
+// is open once they reach r * gridDim.x. One release-add per CTA, then polling with acquire loads.
+//
+// A CTA that met an error in the phase adds it to its arrival, in one of two fields by the barrier's
+// parity; every CTA that passes the barrier sees it there and stops. (A CTA can be one barrier ahead
+// of a slow poller, never two, so the poller's own field holds its own barrier's errors only.)
 //
 // A wait that outlasts `limit` polls breaks the barrier instead of walking away from it: a
-// compare-and-swap sets kBarrierBroken in the counter, and succeeds only if the counter has not
-// moved since it was read. Every CTA therefore agrees on each barrier: either it opened (the last
-// arrival came before the swap) and all pass it, or it is broken and none does -- later arrivals
-// and pollers see the flag and return. The breaker sets ST_TIMEOUT. Since the state is written
-// only in phases that follow an open barrier, a timeout leaves it at the last completed step.
-constexpr unsigned long long kBarrierBroken = 1ull << 62;
-__device__ bool grid_barrier(unsigned long long *arrivals, unsigned long long open_at,
-                             int *status, uint32_t limit) {
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();  // this CTA's writes, ordered by the __syncthreads, before its arrival
-        unsigned long long now = atomicAdd(arrivals, 1ull) + 1ull;
-        ok = 1;
-        uint32_t it = 0;
-        for (;;) {
-            if (now & kBarrierBroken) {
-                ok = 0;
-                break;
-            }
-            if (now >= open_at)
-                break;
-            if (it >= limit) {
-                const unsigned long long seen = atomicCAS(arrivals, now, now | kBarrierBroken);
-                if (seen == now) {
-                    set_status(status, ST_TIMEOUT);
+// compare-and-swap sets the broken flag of the barrier's parity in the counter, and succeeds only if
+// the counter has not moved since it was read. Every CTA therefore agrees on each barrier: either it
+// opened (the last arrival came before the swap) and all pass it -- also a slow poller that finds
+// the next one broken -- or it is broken and none does: later arrivals and pollers see the flag and
+// return. The breaker sets ST_TIMEOUT. Since the state is written only in phases that follow an
+// open barrier, a timeout leaves it at the last completed step.
+constexpr unsigned long long kBarrierCount = (1ull << 40) - 1;
+// errors: 11 bits each from bit 40 and from bit 51, so at most 2047 CTAs
+struct GridBarrier {
+    unsigned long long *arrivals;
+    int *status;
+    uint32_t limit;
+    unsigned long long open_at;  // of the next barrier
+    unsigned parity;
+
+    // Returns true when the barrier opened and no CTA arrived with an error. bad: this thread met one.
+    __device__ __forceinline__ bool wait(bool bad) {
+        __shared__ int go;
+        const int any_bad = __syncthreads_or(bad);
+        open_at += gridDim.x;
+        parity ^= 1u;
+        if (threadIdx.x == 0) {
+            const int shift = parity ? 51 : 40;
+            const unsigned long long broken = parity ? 1ull << 63 : 1ull << 62;
+            const unsigned long long mine = 1ull + (any_bad ? 1ull << shift : 0ull);
+            // this CTA's writes, ordered by the __syncthreads, before its arrival
+            asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(arrivals), "l"(mine)
+                         : "memory");
+            unsigned long long now;
+            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(arrivals) : "memory");
+            int ok = 1;
+            for (uint32_t it = 0;;) {
+                if (now & broken) {
                     ok = 0;
                     break;
                 }
-                now = seen;  // another CTA arrived (or broke it) meanwhile: look again
-                continue;
+                if ((now & kBarrierCount) >= open_at)
+                    break;
+                if (it >= limit) {
+                    const unsigned long long seen = atomicCAS(arrivals, now, now | broken);
+                    if (seen == now) {
+                        set_status(status, ST_TIMEOUT);
+                        ok = 0;
+                        break;
+                    }
+                    now = seen;  // another CTA arrived (or broke it) meanwhile: look again
+                    continue;
+                }
+                ++it;
+                if (it > 256)
+                    __nanosleep(32);
+                asm volatile("ld.acquire.gpu.global.u64 %0, [%1];"
+                             : "=l"(now)
+                             : "l"(arrivals)
+                             : "memory");
             }
-            ++it;
-            if (it > 64)
-                __nanosleep(32);
-            asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(arrivals) : "memory");
+            if (ok && ((now >> shift) & 0x7ffull))
+                ok = 0;
+            go = ok;
         }
-        __threadfence();  // the other CTAs' writes before their arrivals are visible from here
+        __syncthreads();
+        return go != 0;
+    }
+};
+
+// Sources whose pair chains overlap in a thread's chunk sum.
+template <class Pair> struct ChunkUnroll { static constexpr int value = 4; };
+template <> struct ChunkUnroll<InfinitePair> { static constexpr int value = 16; };
+template <> struct ChunkUnroll<DiskPair> { static constexpr int value = 8; };
+
+constexpr int kStepThreads = 256;
+
+// Shared memory of a CTA: all sources, its targets' chunk sums, and per target what its finish
+// keeps from stage to stage.
+struct StepShared {
+    double *x, *y, *g;    // [n]
+    double *qu, *qv;      // [targets][chunks]
+    double *k;            // [7][2][targets]: stage velocities
+    double *x0, *y0;      // [targets]: the step's start
+    __device__ __forceinline__ StepShared(double *base, size_t n, size_t targets, int chunks) {
+        const size_t np = (n + 1) & ~static_cast<size_t>(1);
+        x = base;
+        y = x + np;
+        g = y + np;
+        qu = g + np;
+        qv = qu + targets * chunks;
+        k = qv + targets * chunks;
+        x0 = k + 14 * targets;
+        y0 = x0 + targets;
+    }
+};
+size_t step_shared_bytes(size_t n, size_t targets, int chunks) {
+    const size_t np = (n + 1) & ~static_cast<size_t>(1);
+    return (3 * np + 2 * targets * static_cast<size_t>(chunks) + 16 * targets) * sizeof(double);
+}
+
+// One evaluation: positions (px, py) into shared memory, then the chunk sums of the CTA's targets
+// [t0, t0 + mine).
+template <class Pair>
+__device__ __forceinline__ void step_evaluate(const SmallSteps &p, const StepShared &sh,
+                                              const double *px, const double *py, size_t t0,
+                                              int mine) {
+    const int n2 = static_cast<int>(p.n / 2);
+    const double2 *px2 = reinterpret_cast<const double2 *>(px);
+    const double2 *py2 = reinterpret_cast<const double2 *>(py);
+#pragma unroll 4  // the loads of several iterations in flight at once
+    for (int j = threadIdx.x; j < n2; j += kStepThreads) {
+        reinterpret_cast<double2 *>(sh.x)[j] = __ldcg(px2 + j);
+        reinterpret_cast<double2 *>(sh.y)[j] = __ldcg(py2 + j);
+    }
+    if ((p.n & 1) && threadIdx.x == 0) {
+        sh.x[p.n - 1] = __ldcg(px + p.n - 1);
+        sh.y[p.n - 1] = __ldcg(py + p.n - 1);
     }
     __syncthreads();
-    return ok != 0;
+    const int nc = p.num_chunks;
+    for (int w = threadIdx.x; w < mine * nc; w += kStepThreads) {
+        const int li = w % mine, c = w / mine;
+        const int i = static_cast<int>(t0) + li;
+        const int j0 = c * p.chunk, j1 = min(j0 + p.chunk, static_cast<int>(p.n));
+        const double tx = sh.x[i], ty = sh.y[i];
+        double u = 0.0, v = 0.0;
+        // unrolled so that the independent work of several sources overlaps; the sums still take
+        // the sources in index order
+        constexpr int kUnroll = ChunkUnroll<Pair>::value;
+        int j = j0;
+        for (; j + kUnroll <= j1; j += kUnroll) {
+#pragma unroll
+            for (int q = 0; q < kUnroll; ++q)
+                Pair::template pair<true>(p.g, tx, ty, sh.x[j + q], sh.y[j + q], sh.g[j + q],
+                                          i == j + q, u, v);
+        }
+#pragma unroll 2
+        for (; j < j1; ++j)
+            Pair::template pair<true>(p.g, tx, ty, sh.x[j], sh.y[j], sh.g[j], i == j, u, v);
+        sh.qu[li * nc + c] = u;
+        sh.qv[li * nc + c] = v;
+    }
+    __syncthreads();
+}
+
+// The velocity of target li from its chunk sums (the slow path included), kept as stage s's. Returns
+// an error status, or 0.
+__device__ __forceinline__ int step_velocity(const SmallSteps &p, const StepShared &sh, int li,
+                                             size_t i, int targets, int s) {
+    double ku, kv;
+    const double *qu = sh.qu + li * p.num_chunks, *qv = sh.qv + li * p.num_chunks;
+    sum_chunks(
+        p.num_chunks,
+        [&](int c, double &ru, double &rv) {
+            ru = qu[c];
+            rv = qv[c];
+        },
+        ku, kv);
+    int verdict = 0;
+    if (!isfinite(ku) || !isfinite(kv))  // recomputed from this phase's positions
+        verdict = slow_target(p.g, sh.x, sh.y, p.gamma, p.n, i, ku, kv);
+    sh.k[(2 * s) * targets + li] = ku;
+    sh.k[(2 * s + 1) * targets + li] = kv;
+    return verdict;
+}
+
+// Stage position x0 + dt sum_j a_j k_j of component `part` (makeStage, src/timestep.cpp:19-30).
+__device__ __forceinline__ double step_position(const StepShared &sh, const double *row, int ncoef,
+                                                int part, int li, int targets, double x0,
+                                                double dt) {
+    double d = 0.0;
+    for (int j = 0; j < ncoef; ++j)
+        if (row[j] != 0.0)
+            d = __dadd_rn(d, __dmul_rn(row[j], sh.k[(2 * j + part) * targets + li]));
+    return __dadd_rn(x0, __dmul_rn(dt, d));
 }
 
 template <class Pair>
-__global__ void __launch_bounds__(256) rk4_steps_kernel(const Rk4Steps p) {
-    extern __shared__ double smem[];
-    const size_t n = p.n;
-    const int nc = p.num_chunks;
-    const size_t per_cta = (n + gridDim.x - 1) / gridDim.x;
-    const size_t t0 = static_cast<size_t>(blockIdx.x) * per_cta;
-    const size_t t1 = t0 < n ? min(t0 + per_cta, n) : t0;
-    const int mine = static_cast<int>(t1 - t0);
-    double *sx = smem, *sy = smem + n, *sg = smem + 2 * n;
-    double *qu = smem + 3 * n, *qv = qu + per_cta * nc;
-    int *status = &p.stage[0].ctl->status;
-    for (size_t j = threadIdx.x; j < n; j += blockDim.x)
-        sg[j] = p.gs[j];
-    double local_max = 0.0;
-    unsigned long long open_at = 0;
+__global__ void __launch_bounds__(kStepThreads, 1) rk4_steps_kernel(const SmallSteps p) {
+    extern __shared__ __align__(16) double smem[];
+    const int targets = static_cast<int>((p.n + gridDim.x - 1) / gridDim.x);
+    const size_t t0 = static_cast<size_t>(blockIdx.x) * targets;
+    const int mine = t0 < p.n ? static_cast<int>(min(static_cast<size_t>(targets), p.n - t0)) : 0;
+    const StepShared sh(smem, p.n, targets, p.num_chunks);
+    for (size_t j = threadIdx.x; j < p.n; j += kStepThreads)
+        sh.g[j] = p.gs[j];
+    GridBarrier barrier{&p.ctl->arrivals, &p.ctl->status, p.spin_limit, 0ull, 0u};
+    const int li = threadIdx.x;  // a target's finish is its own thread's
+    const size_t i = t0 + li;
     for (uint64_t step = 0; step < p.steps; ++step) {
-#pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const StageArgs &a = p.stage[s];
             // evaluation point: the state, or for a step's first stage after the first step the
-            // previous step's combination (not yet copied into the state)
-            const bool carried = s == 0 && step > 0;
-            const double *px = carried ? p.stage[3].xt : a.ex;
-            const double *py = carried ? p.stage[3].yt : a.ey;
-#pragma unroll 8  // the loads of several iterations in flight at once
-            for (size_t j = threadIdx.x; j < n; j += blockDim.x) {
-                sx[j] = __ldcg(px + j);
-                sy[j] = __ldcg(py + j);
-            }
-            __syncthreads();
-            for (int w = threadIdx.x; w < mine * nc; w += blockDim.x) {
-                const int li = w % mine, c = w / mine;
-                const size_t i = t0 + li;
-                const size_t j0 = static_cast<size_t>(c) * p.chunk;
-                const size_t j1 = min(j0 + static_cast<size_t>(p.chunk), n);
-                const double tx = sx[i], ty = sy[i];
-                double u = 0.0, v = 0.0;
-                // unrolled so that the independent work of several sources overlaps; the sums
-                // still take the sources in index order
-#pragma unroll 4
-                for (size_t j = j0; j < j1; ++j)
-                    Pair::template pair<true>(a.g, tx, ty, sx[j], sy[j], sg[j], i == j, u, v);
-                qu[li * nc + c] = u;
-                qv[li * nc + c] = v;
-            }
-            __syncthreads();
-            for (int li = threadIdx.x; li < mine; li += blockDim.x) {
-                const size_t i = t0 + li;
-                if (carried) {  // the accept of the previous step
-                    p.x[i] = px[i];
-                    p.y[i] = py[i];
+            // previous step's combination (not yet copied into the state); then the last stage's
+            const double *px = s == 0 ? (step > 0 ? p.px[1] : p.x) : p.px[(s - 1) & 1];
+            const double *py = s == 0 ? (step > 0 ? p.py[1] : p.y) : p.py[(s - 1) & 1];
+            step_evaluate<Pair>(p, sh, px, py, t0, mine);
+            int error = 0;
+            if (li < mine) {
+                if (s == 0) {
+                    sh.x0[li] = sh.x[i];
+                    sh.y0[li] = sh.y[i];
+                    if (step > 0) {  // the accept of the previous step
+                        p.x[i] = sh.x[i];
+                        p.y[i] = sh.y[i];
+                    }
                 }
-                double ku = 0.0, kv = 0.0;
-                for (int c = 0; c < nc; ++c) {
-                    ku += qu[li * nc + c];
-                    kv += qv[li * nc + c];
-                }
-                // the slow path recomputes from this phase's positions, held in shared memory
-                FinishInputs in;
+                error = step_velocity(p, sh, li, i, targets, s);
+                double nx, ny;
                 if (s < 3) {
-                    load_finish_inputs<STAGE_POSITION>(a, i, in);
-                    finish_target<STAGE_POSITION>(a, i, ku, kv, a.dt, local_max, sx, sy, in);
+                    nx = step_position(sh, p.rows[s + 1], s + 1, 0, li, targets, sh.x0[li], p.dt);
+                    ny = step_position(sh, p.rows[s + 1], s + 1, 1, li, targets, sh.y0[li], p.dt);
+                    error = max(error, position_error(p.g, nx, ny));
                 } else {
-                    load_finish_inputs<STAGE_RK4_COMBINE>(a, i, in);
-                    finish_target<STAGE_RK4_COMBINE>(a, i, ku, kv, a.dt, local_max, sx, sy, in);
+                    const double *k = sh.k + li;
+                    nx = rk4_point(sh.x0[li], p.dt, k[0], k[2 * targets], k[4 * targets],
+                                   k[6 * targets]);
+                    ny = rk4_point(sh.y0[li], p.dt, k[targets], k[3 * targets], k[5 * targets],
+                                   k[7 * targets]);
+                    if (!isfinite(nx) || !isfinite(ny))
+                        error = max(error, static_cast<int>(ST_NONFINITE_POSITION));
                 }
+                p.px[s & 1][i] = nx;
+                p.py[s & 1][i] = ny;
+                if (error)
+                    set_status(&p.ctl->status, error);
             }
-            open_at += gridDim.x;
-            if (!grid_barrier(p.barrier, open_at, status, p.spin_limit))
-                return;
-            // every CTA reads the same word after an open barrier: errors are set before arrival
-            if (*reinterpret_cast<volatile int *>(status) != 0)
+            if (!barrier.wait(error != 0))
                 return;
         }
     }
-    for (int li = threadIdx.x; li < mine; li += blockDim.x) {  // the last step's accept
-        const size_t i = t0 + li;
-        p.x[i] = __ldcg(p.stage[3].xt + i);
-        p.y[i] = __ldcg(p.stage[3].yt + i);
+    if (li < mine) {  // the last step's accept
+        p.x[i] = __ldcg(p.px[1] + i);
+        p.y[i] = __ldcg(p.py[1] + i);
     }
 }
 
-size_t rk4_steps_smem(size_t n, int num_chunks, int grid) {
-    const size_t per_cta = (n + grid - 1) / grid;
-    return (3 * n + 2 * per_cta * static_cast<size_t>(num_chunks)) * sizeof(double);
-}
-
-bool rk4_steps_eligible(size_t n, int num_chunks) {
-    return n >= 1 && n <= kRk4StepsMaxN && num_chunks >= 1 && num_chunks < kWideRows;
-}
-
+// One adaptive step (src/timestep.cpp:62-120). need_k0: the derivative at the state is not cached in
+// (k0x, k0y). A rejected attempt changes only the step size, so the next one starts from the same
+// k0 without leaving the kernel; an accepted one updates the state and k0.
 template <class Pair>
-cudaError_t launch_rk4_steps_t(const Rk4Steps &p, int grid, cudaStream_t stream) {
-    const size_t smem = rk4_steps_smem(p.n, p.num_chunks, grid);
-    cudaError_t e = cudaFuncSetAttribute(rk4_steps_kernel<Pair>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+__global__ void __launch_bounds__(kStepThreads, 1) dopri_step_kernel(const SmallSteps p) {
+    extern __shared__ __align__(16) double smem[];
+    __shared__ double s_error;
+    const int targets = static_cast<int>((p.n + gridDim.x - 1) / gridDim.x);
+    const size_t t0 = static_cast<size_t>(blockIdx.x) * targets;
+    const int mine = t0 < p.n ? static_cast<int>(min(static_cast<size_t>(targets), p.n - t0)) : 0;
+    const StepShared sh(smem, p.n, targets, p.num_chunks);
+    for (size_t j = threadIdx.x; j < p.n; j += kStepThreads)
+        sh.g[j] = p.gs[j];
+    GridBarrier barrier{&p.ctl->arrivals, &p.ctl->status, p.spin_limit, 0ull, 0u};
+    const int li = threadIdx.x;
+    const size_t i = t0 + li;
+    const bool owner = li < mine;
+    DeviceControl *ctl = p.ctl;
+    const double minimum = ctl->minimum_time_step, maximum = ctl->maximum_time_step;
+    double dt = ctl->dt;
+    unsigned rejected = 0;
+    if (owner) {
+        sh.x0[li] = p.x[i];
+        sh.y0[li] = p.y[i];
+        if (!p.need_k0) {
+            sh.k[li] = p.k0x[i];
+            sh.k[targets + li] = p.k0y[i];
+        }
+    }
+    for (int attempt = 0;; ++attempt) {
+        // the error words alternate; this attempt's was last read two attempts ago
+        unsigned long long *word = attempt & 1 ? &ctl->err_bits2 : &ctl->err_bits;
+        if (attempt > 0 && blockIdx.x == 0 && threadIdx.x == 0)
+            *word = 0ull;
+        double x5 = 0.0, y5 = 0.0, local = 0.0;
+        for (int s = 0; s < 7; ++s) {
+            const bool evaluate = s > 0 || (p.need_k0 && attempt == 0);
+            if (evaluate)
+                step_evaluate<Pair>(p, sh, s == 0 ? p.x : p.px[(s - 1) & 1],
+                                    s == 0 ? p.y : p.py[(s - 1) & 1], t0, mine);
+            int error = 0;
+            if (owner) {
+                if (evaluate)
+                    error = step_velocity(p, sh, li, i, targets, s);
+                if (s < 6) {
+                    x5 = step_position(sh, p.rows[s + 1], s + 1, 0, li, targets, sh.x0[li], dt);
+                    y5 = step_position(sh, p.rows[s + 1], s + 1, 1, li, targets, sh.y0[li], dt);
+                    p.px[s & 1][i] = x5;
+                    p.py[s & 1][i] = y5;
+                    error = max(error, position_error(p.g, x5, y5));
+                } else {  // (x5, y5): the fifth-order point, the position of k6
+                    double xe = 0.0, ye = 0.0;
+                    for (int j = 0; j < 7; ++j) {
+                        if (p.w[j] == 0.0)
+                            continue;
+                        const double h = __dmul_rn(dt, p.w[j]);
+                        xe = __dadd_rn(xe, __dmul_rn(h, sh.k[(2 * j) * targets + li]));
+                        ye = __dadd_rn(ye, __dmul_rn(h, sh.k[(2 * j + 1) * targets + li]));
+                    }
+                    const double xs = error_scale(ctl, sh.x0[li], x5);
+                    const double ys = error_scale(ctl, sh.y0[li], y5);
+                    if (!isfinite(xe) || !isfinite(ye) || !isfinite(xs) || !isfinite(ys) ||
+                        !(xs > 0.0) || !(ys > 0.0))
+                        error = max(error, static_cast<int>(ST_DOPRI_NONFINITE));
+                    else
+                        local = max_ref(__ddiv_rn(fabs(xe), xs), __ddiv_rn(fabs(ye), ys));
+                }
+                if (error)
+                    set_status(&ctl->status, error);
+            }
+            if (s == 6 && threadIdx.x < 32 * ((mine + 31) / 32)) {  // whole warps of owners
+                for (int off = 16; off > 0; off >>= 1)
+                    local = max_ref(local, __shfl_xor_sync(0xffffffffu, local, off));
+                if ((threadIdx.x & 31) == 0)
+                    atomicMax(word, ordered_bits(local));
+            }
+            if (!barrier.wait(error != 0)) {
+                if (blockIdx.x == 0 && threadIdx.x == 0)
+                    ctl->attempts = attempt + 1;
+                return;
+            }
+        }
+        if (threadIdx.x == 0)
+            s_error = __longlong_as_double(
+                static_cast<long long>(*reinterpret_cast<volatile unsigned long long *>(word)));
+        __syncthreads();
+        // every thread takes the same decision from the same numbers
+        const double error = s_error;
+        int accepted;
+        double suggested, next_dt;
+        const int failed =
+            dopri_decide(error, dt, minimum, maximum, rejected, accepted, suggested, next_dt);
+        if (accepted && owner) {
+            p.x[i] = x5;
+            p.y[i] = y5;
+            p.k0x[i] = sh.k[12 * targets + li];
+            p.k0y[i] = sh.k[13 * targets + li];
+        }
+        if ((accepted || failed) && blockIdx.x == 0 && threadIdx.x == 0) {
+            ctl->accepted = accepted;
+            ctl->rejected = rejected;
+            ctl->attempts = attempt + 1;
+            if (accepted)
+                store_accepted(ctl, dt, suggested, error, rejected);
+            else
+                set_status(&ctl->status, failed);
+        }
+        if (accepted || failed)
+            return;
+        dt = next_dt;
+    }
+}
+
+bool small_steps_eligible(size_t n, int num_chunks, int sm_count) {
+    const size_t grid = static_cast<size_t>(sm_count > 0 ? sm_count : 148);
+    return n >= 1 && n <= kSmallStepsMaxN && num_chunks >= 1 && num_chunks < kWideRows &&
+           grid <= 2047 && (n + grid - 1) / grid <= kStepThreads;
+}
+
+namespace {
+template <class Kernel>
+cudaError_t launch_cooperative(Kernel kernel, const SmallSteps &p, int sm_count,
+                               cudaStream_t stream) {
+    const size_t grid =
+        std::min<size_t>(static_cast<size_t>(sm_count > 0 ? sm_count : 148), p.n);
+    const size_t smem = step_shared_bytes(p.n, (p.n + grid - 1) / grid, p.num_chunks);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
     if (e != cudaSuccess)
         return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(static_cast<unsigned>(grid));
-    cfg.blockDim = dim3(256);
+    cfg.blockDim = dim3(kStepThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -661,22 +940,27 @@ cudaError_t launch_rk4_steps_t(const Rk4Steps &p, int grid, cudaStream_t stream)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, rk4_steps_kernel<Pair>, p);
+    return cudaLaunchKernelEx(&cfg, kernel, p);
 }
 
-cudaError_t launch_rk4_steps(const Rk4Steps &p, int sm_count, cudaStream_t stream) {
-    if (!rk4_steps_eligible(p.n, p.num_chunks) || p.steps == 0 || !p.barrier)
+template <class Pair>
+cudaError_t launch_small(const SmallSteps &p, int sm_count, cudaStream_t stream) {
+    return p.dopri ? launch_cooperative(dopri_step_kernel<Pair>, p, sm_count, stream)
+                   : launch_cooperative(rk4_steps_kernel<Pair>, p, sm_count, stream);
+}
+} // namespace
+
+cudaError_t launch_small_steps(const SmallSteps &p, int sm_count, cudaStream_t stream) {
+    if (!small_steps_eligible(p.n, p.num_chunks, sm_count) || (!p.dopri && p.steps == 0))
         return cudaErrorInvalidValue;
-    const int grid = static_cast<int>(
-        std::min<size_t>(static_cast<size_t>(sm_count > 0 ? sm_count : 148), p.n));
-    switch (p.stage[0].g.geometry) {
+    switch (p.g.geometry) {
     case GEO_INFINITE:
-        return launch_rk4_steps_t<InfinitePair>(p, grid, stream);
+        return launch_small<InfinitePair>(p, sm_count, stream);
     case GEO_PERIODIC:
-        return p.stage[0].g.zeta ? launch_rk4_steps_t<ZetaPair>(p, grid, stream)
-                                 : launch_rk4_steps_t<PeriodicPair>(p, grid, stream);
+        return p.g.zeta ? launch_small<ZetaPair>(p, sm_count, stream)
+                        : launch_small<PeriodicPair>(p, sm_count, stream);
     case GEO_DISK:
-        return launch_rk4_steps_t<DiskPair>(p, grid, stream);
+        return launch_small<DiskPair>(p, sm_count, stream);
     default:
         return cudaErrorInvalidValue;
     }

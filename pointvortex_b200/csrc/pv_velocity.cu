@@ -253,6 +253,12 @@ EvalPlan plan_evaluation(const GeometryConsts &g, size_t n_targets, size_t n_sou
     if (blocks_of(p.per_thread) * std::max<size_t>(1, n_sources / min_chunk) <
         sms * resident_of(p.per_thread))
         min_chunk = 64;
+    // Small FP64 populations are bound by the serial sum over a chunk (one source after another):
+    // chunks down to 24 sources, but fewer than 32 of them (the cooperative steps and the narrow
+    // reduction).
+    const bool small = precision == 0 && n_sources <= kSmallStepsMaxN;
+    if (small)
+        min_chunk = 24;
     p.target_blocks = static_cast<int>(blocks_of(p.per_thread));
     const size_t slots = sms * resident_of(p.per_thread);
     const size_t max_chunks = std::max<size_t>(1, n_sources / min_chunk);
@@ -260,7 +266,8 @@ EvalPlan plan_evaluation(const GeometryConsts &g, size_t n_targets, size_t n_sou
     // count (up to four waves) whose last wave is fullest; ties go to fewer chunks.
     size_t best_chunks = 1;
     double best_eff = -1.0;
-    const size_t limit = std::min<size_t>(max_chunks, std::max<size_t>(1, 4 * slots / p.target_blocks + 1));
+    const size_t limit = std::min<size_t>(std::min<size_t>(max_chunks, small ? 31 : max_chunks),
+                                          std::max<size_t>(1, 4 * slots / p.target_blocks + 1));
     for (size_t c = 1; c <= limit; ++c) {
         const size_t chunk = std::max<size_t>(2, ((n_sources + c - 1) / c + 1) & ~size_t(1));
         const size_t chunks = (n_sources + chunk - 1) / chunk;
