@@ -903,10 +903,28 @@ __global__ void __launch_bounds__(256) batch_accept_kernel(const SliceEntry *sli
     arena.ky[0][e] = arena.ky[6][e];
 }
 
-__global__ void scale_kernel(const double *gamma, double *gs, size_t n, GeometryConsts g) {
-    for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<size_t>(gridDim.x) * blockDim.x)
-        gs[i] = scaled_circulation(g, gamma[i]);
+// Admission: x, y and circulation (n doubles each, one after another at src) into the arena, the
+// scaled circulations, and the slot's descriptor and control, which follow them at src.
+__global__ void __launch_bounds__(256)
+    admit_kernel(const double *src, size_t n, double *x, double *y, double *gamma, double *gs,
+                 SimDesc *desc, SimControl *ctl) {
+    const SimDesc *d = reinterpret_cast<const SimDesc *>(src + 3 * n);
+    const SimControl *c = reinterpret_cast<const SimControl *>(d + 1);
+    const size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
+    if (i < n) {
+        x[i] = src[i];
+        y[i] = src[n + i];
+        const double g = src[2 * n + i];
+        gamma[i] = g;
+        gs[i] = scaled_circulation(d->g, g);
+    }
+    if (blockIdx.x == 0) {
+        static_assert(sizeof(SimDesc) % 8 == 0 && sizeof(SimControl) % 8 == 0, "copied by doubles");
+        for (unsigned k = threadIdx.x; k < sizeof(SimDesc) / 8; k += blockDim.x)
+            reinterpret_cast<double *>(desc)[k] = reinterpret_cast<const double *>(d)[k];
+        for (unsigned k = threadIdx.x; k < sizeof(SimControl) / 8; k += blockDim.x)
+            reinterpret_cast<double *>(ctl)[k] = reinterpret_cast<const double *>(c)[k];
+    }
 }
 
 size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
@@ -927,13 +945,17 @@ struct pv_batch {
     void *arena_block = nullptr;
     SimDesc *d_descs = nullptr;
     SimControl *d_ctl = nullptr;
-    SimControl *h_ctl = nullptr;       // pinned mirror
+    SimControl *h_ctl = nullptr;       // pinned mirror, behind h_stage's bytes
     Item *d_items = nullptr;
     size_t items_cap = 0;
     SliceEntry *d_slices = nullptr;
     size_t slices_cap = 0;
     unsigned *d_counters = nullptr;    // one queue counter per velocity launch of an attempt
     int *d_timeout = nullptr;
+    // pinned staging and its device twin, handed out front to back (stage()): an admission is one
+    // copy and one kernel, and several may be in flight
+    char *h_stage = nullptr, *d_stage = nullptr;
+    size_t stage_used = 0;
     int resident = 1;                  // FP64 velocity CTAs per SM
     int resident32 = 1;                // FP32C velocity CTAs per SM
     std::vector<SimDesc> descs;
@@ -958,11 +980,12 @@ struct pv_batch {
         cudaFree(arena_block);
         cudaFree(d_descs);
         cudaFree(d_ctl);
-        cudaFreeHost(h_ctl);
         cudaFree(d_items);
         cudaFree(d_slices);
         cudaFree(d_counters);
         cudaFree(d_timeout);
+        cudaFreeHost(h_stage);
+        cudaFree(d_stage);
         if (stream)
             cudaStreamDestroy(stream);
     }
@@ -981,6 +1004,19 @@ pv_status bfail(pv_batch *b, pv_status code, const std::string &m) {
         if (e_ != cudaSuccess)                                                                     \
             return bfail((b), PV_ERROR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_));  \
     } while (0)
+
+constexpr size_t kStageBytes = static_cast<size_t>(256) << 10;  // pinning more is felt at creation
+
+// Offset of `bytes` of staging that no copy in flight uses.
+pv_status stage(pv_batch *b, size_t bytes, size_t &off) {
+    if (b->stage_used + bytes > kStageBytes) {
+        PVB_CUDA(b, cudaStreamSynchronize(b->stream));
+        b->stage_used = 0;
+    }
+    off = b->stage_used;
+    b->stage_used += round_up(bytes, 256);
+    return PV_OK;
+}
 
 bool take(std::map<size_t, size_t> &free, size_t len, size_t &off) {
     for (auto it = free.begin(); it != free.end(); ++it)
@@ -1260,10 +1296,12 @@ pv_status pv_batch_create(const pv_batch_config *config, pv_batch **out) {
     b->arena.pv = next(b->part_capacity);
     if ((e = cudaMalloc(&b->d_descs, b->max_sims * sizeof(SimDesc))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_ctl, b->max_sims * sizeof(SimControl))) != cudaSuccess ||
-        (e = cudaMallocHost(&b->h_ctl, b->max_sims * sizeof(SimControl))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_counters, kCounters * sizeof(unsigned))) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_timeout, sizeof(int))) != cudaSuccess)
+        (e = cudaMalloc(&b->d_timeout, sizeof(int))) != cudaSuccess ||
+        (e = cudaMallocHost(&b->h_stage, kStageBytes + b->max_sims * sizeof(SimControl))) != cudaSuccess ||
+        (e = cudaMalloc(&b->d_stage, kStageBytes)) != cudaSuccess)
         return bail(e, "cudaMalloc(batch tables)");
+    b->h_ctl = reinterpret_cast<SimControl *>(b->h_stage + kStageBytes);
     std::memset(b->h_ctl, 0, b->max_sims * sizeof(SimControl));
     cudaMemcpy(b->d_ctl, b->h_ctl, b->max_sims * sizeof(SimControl), cudaMemcpyHostToDevice);
     cudaMemset(b->d_timeout, 0, sizeof(int));
@@ -1370,19 +1408,27 @@ pv_status pv_batch_add(pv_batch *b, const pv_params *params, const double *x, co
     if (c.t_end <= 0.0)
         c.state = SIM_DONE;
     cudaSetDevice(b->device);
-    const size_t bytes = n * sizeof(double);
-    PVB_CUDA(b, cudaMemcpyAsync(b->arena.x + off, x, bytes, cudaMemcpyHostToDevice, b->stream));
-    PVB_CUDA(b, cudaMemcpyAsync(b->arena.y + off, y, bytes, cudaMemcpyHostToDevice, b->stream));
-    PVB_CUDA(b, cudaMemcpyAsync(b->arena.gamma + off, circulation, bytes, cudaMemcpyHostToDevice, b->stream));
-    scale_kernel<<<(static_cast<unsigned>(n) + 255) / 256, 256, 0, b->stream>>>(b->arena.gamma + off,
-                                                                                b->arena.gs + off, n, g);
-    PVB_CUDA(b, cudaGetLastError());
-    PVB_CUDA(b, cudaMemcpyAsync(b->d_descs + slot, &b->descs[slot], sizeof(SimDesc),
-                                cudaMemcpyHostToDevice, b->stream));
     b->h_ctl[slot] = c;
-    PVB_CUDA(b, cudaMemcpyAsync(b->d_ctl + slot, &b->h_ctl[slot], sizeof(SimControl),
-                                cudaMemcpyHostToDevice, b->stream));
-    PVB_CUDA(b, cudaStreamSynchronize(b->stream));
+    const size_t tail = sizeof(SimDesc) + sizeof(SimControl);
+    const size_t most = (kStageBytes - tail) / (3 * sizeof(double));
+    for (size_t from = 0; from < n; from += most) {
+        const size_t count = std::min(most, n - from), bytes = count * sizeof(double);
+        size_t at = 0;
+        if ((st = stage(b, 3 * bytes + tail, at)) != PV_OK)
+            return st;
+        char *host = b->h_stage + at, *dev = b->d_stage + at;
+        std::memcpy(host, x + from, bytes);
+        std::memcpy(host + bytes, y + from, bytes);
+        std::memcpy(host + 2 * bytes, circulation + from, bytes);
+        std::memcpy(host + 3 * bytes, &d, sizeof(SimDesc));
+        std::memcpy(host + 3 * bytes + sizeof(SimDesc), &c, sizeof(SimControl));
+        PVB_CUDA(b, cudaMemcpyAsync(dev, host, 3 * bytes + tail, cudaMemcpyHostToDevice, b->stream));
+        const size_t to = off + from;
+        admit_kernel<<<static_cast<unsigned>((count + 255) / 256), 256, 0, b->stream>>>(
+            reinterpret_cast<const double *>(dev), count, b->arena.x + to, b->arena.y + to,
+            b->arena.gamma + to, b->arena.gs + to, b->d_descs + slot, b->d_ctl + slot);
+        PVB_CUDA(b, cudaGetLastError());
+    }
     b->slot_used[slot] = c.state;
     b->tables_dirty = true;
     *id = slot;
@@ -1419,6 +1465,7 @@ pv_status pv_batch_advance(pv_batch *b, uint32_t attempts, uint32_t *running) {
     PVB_CUDA(b, cudaMemcpyAsync(b->h_ctl, b->d_ctl, b->max_sims * sizeof(SimControl),
                                 cudaMemcpyDeviceToHost, b->stream));
     PVB_CUDA(b, cudaStreamSynchronize(b->stream));
+    b->stage_used = 0;
     int timeout = 0;
     PVB_CUDA(b, cudaMemcpy(&timeout, b->d_timeout, sizeof(int), cudaMemcpyDeviceToHost));
     if (timeout)
@@ -1478,9 +1525,25 @@ pv_status pv_batch_result(pv_batch *b, uint32_t id, double *x, double *y, size_t
         return bfail(b, PV_ERROR_RUNTIME, "host and device vortex populations differ");
     cudaSetDevice(b->device);
     const size_t off = b->descs[id].off;
-    PVB_CUDA(b, cudaMemcpyAsync(x, b->arena.x + off, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
-    PVB_CUDA(b, cudaMemcpyAsync(y, b->arena.y + off, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
+    const size_t bytes = n * sizeof(double);
+    const bool staged = 2 * bytes <= kStageBytes;
+    size_t at = 0;
+    if (staged) {
+        const pv_status st = stage(b, 2 * bytes, at);
+        if (st != PV_OK)
+            return st;
+    }
+    char *host = b->h_stage + at;
+    PVB_CUDA(b, cudaMemcpyAsync(staged ? static_cast<void *>(host) : x, b->arena.x + off, bytes,
+                                cudaMemcpyDeviceToHost, b->stream));
+    PVB_CUDA(b, cudaMemcpyAsync(staged ? static_cast<void *>(host + bytes) : y, b->arena.y + off,
+                                bytes, cudaMemcpyDeviceToHost, b->stream));
     PVB_CUDA(b, cudaStreamSynchronize(b->stream));
+    b->stage_used = 0;
+    if (staged) {
+        std::memcpy(x, host, bytes);
+        std::memcpy(y, host + bytes, bytes);
+    }
     return PV_OK;
 }
 

@@ -245,10 +245,18 @@ class VelocityKernel:
     # -- text output formatted on the GPU (the reference's setprecision(17) streams) ----------
     def _formatted(self, call, n_rows: int, row_max: int) -> bytes:
         cap = max(n_rows * row_max, 1)
-        buf = ctypes.create_string_buffer(cap)
+        # A buffer of up to 32 MB is kept between calls, since the fresh pages of a frame cost more than
+        # its copy; a call takes it away meanwhile, so two threads never share it.
+        buf = self.__dict__.pop("_text", None)
+        if buf is None or buf.size < cap:
+            buf = np.empty(cap, dtype=np.uint8)
+        at = buf.ctypes.data
         length = ctypes.c_size_t(0)
-        self._check(call(buf, cap, ctypes.byref(length)))
-        return buf.raw[:length.value]
+        self._check(call(ctypes.cast(at, ctypes.c_char_p), cap, ctypes.byref(length)))
+        text = ctypes.string_at(at, length.value)
+        if buf.size <= 32 << 20:
+            self._text = buf
+        return text
 
     def formatTrajectory(self, time: float, frame: int) -> bytes:
         """The rows TrajectoryWriter::write (src/print.cpp:29-40) appends for the device state,
