@@ -133,7 +133,7 @@ struct pv_context {
     unsigned long long prescan_count = 0;
 
     // text output (pv_format_*): row slots, row lengths, block offsets, the packed frame
-    DeviceArray fmt_stage, fmt_len, fmt_block, fmt_out;
+    DeviceArray fmt_stage, fmt_block, fmt_out;
 
     // FP32C near field (pv_set_near_field): the lists of pairs left to the FP64 pass, and the
     // radius (< 0: the default for the population, 0: none)
@@ -168,7 +168,7 @@ struct pv_context {
             cudaGraphExecDestroy(attempt_graph);
         for (DeviceArray *a : {&x, &y, &gamma, &gs, &p0x, &p0y, &p1x, &p1y, &pu, &pv, &inv_scratch,
                                &inv_out, &cand, &ex, &ey, &eg, &egs, &eu, &ev, &epu, &epv,
-                               &removed_index, &fmt_stage, &fmt_len, &fmt_block, &fmt_out,
+                               &removed_index, &fmt_stage, &fmt_block, &fmt_out,
                                &sym_items, &sym_counter, &near_count, &near_slot})
             a->release();
         for (int s = 0; s < 7; ++s) {
@@ -1842,17 +1842,15 @@ namespace {
 pv_status format_rows(pv_context *ctx, RowFormat f, char *out, size_t capacity, size_t *length,
                       bool check_velocity) {
     const size_t n = f.n;
-    const size_t blocks = (n + 255) / 256;
+    const size_t blocks = (n + kFormatRows - 1) / kFormatRows;
     auto words = [](size_t bytes) { return (bytes + 7) / 8; };
     PV_CUDA(ctx, ctx->fmt_stage.ensure(words(n * static_cast<size_t>(f.stride))));
     PV_CUDA(ctx, ctx->fmt_out.ensure(words(n * static_cast<size_t>(f.stride))));
-    PV_CUDA(ctx, ctx->fmt_len.ensure(words(n * sizeof(uint32_t))));
     PV_CUDA(ctx, ctx->fmt_block.ensure(blocks + 1));
     char *dev_out = reinterpret_cast<char *>(ctx->fmt_out.p);
     auto *block = reinterpret_cast<unsigned long long *>(ctx->fmt_block.p);
     PV_CUDA(ctx, counted(ctx, PV_KERNEL_OUTPUT, 3, [&] {
-                return launch_format_rows(f, reinterpret_cast<char *>(ctx->fmt_stage.p),
-                                          reinterpret_cast<uint32_t *>(ctx->fmt_len.p), block,
+                return launch_format_rows(f, reinterpret_cast<char *>(ctx->fmt_stage.p), block,
                                           dev_out, ctx->stream);
             }));
     auto *total = reinterpret_cast<unsigned long long *>(ctx->pinned);

@@ -6,12 +6,18 @@
 // value is printed with 17 significant digits, correctly rounded (ties to even) from its exact
 // binary value, in the shorter of the fixed and exponent forms that %g chooses, with trailing
 // zeros removed. Correct rounding needs the exact value, so the scaling by a power of ten is done
-// in integer arithmetic on up to 1152-bit numbers:
+// in integer arithmetic, on up to 1152-bit numbers in general:
 //
 //   |v| = m 2^e (53-bit m), k = floor(log10 |v|), s = 16 - k,
 //   D = round_half_even(|v| 10^s) in [10^16, 10^17]   (D = 10^17 -> D = 10^16, k + 1)
 //   s >= 0:  |v| 10^s = m 5^s 2^(e+s)         (one big product, then a shift)
 //   s <  0:  |v| 10^s = m 2^e / (5^-s 2^-s)   (a 61-bit quotient by binary long division)
+//
+// For 0 <= s <= 27, |v| from about 1e-11 to 1e17, 5^s is below 2^63 and the product below 2^116: two
+// words hold it. What coordinates and velocities of files are goes that way, in registers; the
+// 18-word numbers live in a thread's local memory, which bound a frame's kernels (mean of a trajectory
+// and a checkpoint frame: 16384 rows 119 us, 262144 rows 430 us; with the two-word path and rows
+// collected in shared memory 31 and 95 us). Outside, -11 > log10 |v| or |v| >= 1e17, they still serve.
 //
 // k starts from floor(b log10 2) for the top bit b of |v| ((b * 78913) >> 18, exact for
 // |b| <= 1100) and moves up by one when the scaled value reaches 10^17. The functions are
@@ -22,8 +28,10 @@
 
 #if defined(__CUDACC__)
 #define PVF_HD __host__ __device__ __forceinline__
+#define PVF_HD_CALL inline __host__ __device__ __noinline__
 #else
 #define PVF_HD inline
+#define PVF_HD_CALL inline
 #endif
 
 namespace pvb {
@@ -144,7 +152,7 @@ PVF_HD uint64_t big_bits64(const Big &a, int from) {  // bits [from, from + 64)
 
 // floor(m 2^e 10^s) and where the dropped fraction lies against one half (-1 below, 0 at,
 // +1 above). The quotient is below 2^61 for the s this file uses.
-PVF_HD uint64_t scaled_floor(uint64_t m, int e, int s, int &half_cmp) {
+PVF_HD_CALL uint64_t scaled_floor_big(uint64_t m, int e, int s, int &half_cmp) {
     Big n;
     big_set(n, m);
     if (s >= 0) {
@@ -185,16 +193,69 @@ PVF_HD uint64_t scaled_floor(uint64_t m, int e, int s, int &half_cmp) {
     return q;
 }
 
+PVF_HD uint64_t scaled_floor(uint64_t m, int e, int s, int &half_cmp) {
+    if (s < 0 || s > 27)
+        return scaled_floor_big(m, e, s, half_cmp);
+    uint64_t f = (s & 1) ? 5 : 1;  // 5^s
+    f *= (s & 2) ? 25 : 1;
+    f *= (s & 4) ? 625 : 1;
+    f *= (s & 8) ? 390625 : 1;
+    f *= (s & 16) ? 152587890625ull : 1;
+    uint64_t lo, hi;
+    mul_wide(m, f, lo, hi);
+    const int t = e + s;
+    if (t >= 0) {  // the quotient, below 2^61, is all of it
+        half_cmp = -1;
+        return lo << t;
+    }
+    // Both the product (below 2^116) and the quotient (10^16 / 10 at least, above 2^49) bound the
+    // shift: 1 <= -t <= 66.
+    const int sh = -t;
+    const uint64_t q = sh < 64 ? (lo >> sh) | (hi << 1 << (63 - sh)) : hi >> (sh - 64);
+    const int h = sh - 1;  // the bit of one half; what lies below it
+    const bool half = h < 64 ? (lo >> h) & 1 : (hi >> (h - 64)) & 1;
+    const bool rest = h < 64 ? (lo & ((uint64_t{1} << h) - 1)) != 0
+                             : lo != 0 || (hi & ((uint64_t{1} << (h - 64)) - 1)) != 0;
+    half_cmp = !half ? -1 : (rest ? 1 : 0);
+    return q;
+}
+
 PVF_HD int format_u64(uint64_t v, char *out) {
-    char tmp[kMaxU64Chars];
-    int n = 0;
-    do {
-        tmp[n++] = static_cast<char>('0' + v % 10);
-        v /= 10;
-    } while (v);
-    for (int i = 0; i < n; ++i)
-        out[i] = tmp[n - 1 - i];
+    int n = 1;
+    if (v >> 32) {
+        for (uint64_t p = 10; n < kMaxU64Chars && v >= p; p *= 10)
+            ++n;  // 10^19 is the last power: p wraps only after it
+        for (int i = n - 1; i >= 0; --i) {
+            out[i] = static_cast<char>('0' + v % 10);
+            v /= 10;
+        }
+        return n;
+    }
+    uint32_t w = static_cast<uint32_t>(v);
+    for (uint32_t p = 10; n < 10 && w >= p; p *= 10)
+        ++n;
+    for (int i = n - 1; i >= 0; --i) {
+        out[i] = static_cast<char>('0' + w % 10);
+        w /= 10;
+    }
     return n;
+}
+
+// The digits of w, `count` of them from place `first` on, into out with a gap after place `gap`;
+// returns the place of the last one that is not zero, or `last`.
+template <int COUNT>
+PVF_HD int put_digits(uint32_t w, int first, int gap, char *out, int last) {
+#if defined(__CUDA_ARCH__)
+#pragma unroll
+#endif
+    for (int j = COUNT - 1; j >= 0; --j) {
+        const uint32_t d = w % 10;
+        w /= 10;
+        const int i = first + j;
+        out[i + (i > gap ? 1 : 0)] = static_cast<char>('0' + d);
+        last = last < i && d ? i : last;
+    }
+    return last;
 }
 
 // "%.17g" of v into out (at most kMaxDoubleChars bytes, no terminator); returns the length.
@@ -238,39 +299,28 @@ PVF_HD int format_g17(double v, char *out) {
         q = p16;
         ++k;
     }
-    char dig[17];
-    for (int i = 16; i >= 0; --i) {
-        dig[i] = static_cast<char>('0' + q % 10);
-        q /= 10;
-    }
-    int last = 16;  // last significant digit after trailing zeros go
-    while (last > 0 && dig[last] == '0')
-        --last;
-    if (k >= -4 && k < 17) {
-        if (k >= 0) {
-            for (int i = 0; i <= k; ++i)
-                out[len++] = dig[i];
-            if (last > k) {
-                out[len++] = '.';
-                for (int i = k + 1; i <= last; ++i)
-                    out[len++] = dig[i];
-            }
-        } else {
-            out[len++] = '0';
-            out[len++] = '.';
-            for (int i = 0; i < -k - 1; ++i)
-                out[len++] = '0';
-            for (int i = 0; i <= last; ++i)
-                out[len++] = dig[i];
-        }
-        return len;
-    }
-    out[len++] = dig[0];
-    if (last > 0) {
+    // All 17 digits go to their places, with a gap for the point after place `gap`; trailing zeros
+    // are cut off by the length.
+    const bool fixed = k >= -4 && k < 17;
+    int gap = fixed ? k : 0;
+    if (fixed && k < 0) {
+        out[len++] = '0';
         out[len++] = '.';
-        for (int i = 1; i <= last; ++i)
-            out[len++] = dig[i];
+        for (int i = 0; i < -k - 1; ++i)
+            out[len++] = '0';
+        gap = 16;
     }
+    const uint64_t q8 = q / 100000000u;
+    int last = put_digits<8>(static_cast<uint32_t>(q - q8 * 100000000u), 9, gap, out + len, 0);
+    last = put_digits<9>(static_cast<uint32_t>(q8), 0, gap, out + len, last);
+    if (last > gap) {
+        out[len + gap + 1] = '.';
+        len += last + 2;
+    } else {
+        len += (fixed && k < 0 ? last : gap) + 1;  // with k >= 0 the places before the point stay
+    }
+    if (fixed)
+        return len;
     out[len++] = 'e';
     out[len++] = k < 0 ? '-' : '+';
     const int ak = k < 0 ? -k : k;

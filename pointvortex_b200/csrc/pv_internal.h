@@ -255,10 +255,11 @@ struct RowFormat {
 // "time,frame," as the trajectory rows begin; returns its length (at most 46).
 int format_prefix(double time, uint64_t frame, char *out);
 // Formats rows [0, f.n) into staging (f.stride bytes each), then packs them into out;
-// block_sums needs ceil(n / 256) + 1 entries and receives the frame's byte count at
-// block_sums[ceil(n / 256)].
-cudaError_t launch_format_rows(const RowFormat &f, char *staging, uint32_t *lengths,
-                               unsigned long long *block_sums, char *out, cudaStream_t stream);
+// block_sums needs ceil(n / kFormatRows) + 1 entries and receives the frame's byte count at
+// block_sums[ceil(n / kFormatRows)].
+constexpr int kFormatRows = 128;  // rows of a block
+cudaError_t launch_format_rows(const RowFormat &f, char *staging, unsigned long long *block_sums,
+                               char *out, cudaStream_t stream);
 
 // ---- shared host helpers (pv_context.cu) -------------------------------------------------------
 // Kernel-constructor validation and fast-path constants of a parameter set.
