@@ -388,10 +388,11 @@ __device__ __forceinline__ void periodic_pair(const GeometryConsts &g, double tx
 // The box's pair energy in the same units, -x^2/(2 pi) + sum_m [log D(m) - log cosh(2 pi m)] of the
 // reference (x, y here times 2 pi/L), which is 2 log|sigma(z)| - pi |z|^2/L^2 + constant: sigma is
 // entire, sigma(z)/z a function of z^4 alone, and a polynomial of degree 7 over the box. One logarithm
-// a pair, of |z|^2 |S|^2, and 30 more FP64 instructions; the image product it replaces took two
-// logarithms, both half-angle series and four instructions an image. coincident: z == 0.
+// a pair, of the argument |z|^2 |S|^2 (0 only for z = 0), added to `rest`, and 30 more FP64
+// instructions; the image product it replaces took two logarithms, both half-angle series and four
+// instructions an image.
 __device__ __forceinline__ double box_energy(const GeometryConsts &g, double x, double y,
-                                             bool &coincident) {
+                                             double &rest) {
     const double yy = y * y;
     const double a = fma(x, x, -yy), r = fma(x, x, yy), b = x * y;
     const double r2 = r * r, n = r2 * r2;
@@ -406,8 +407,8 @@ __device__ __forceinline__ double box_energy(const GeometryConsts &g, double x, 
         s1 = s0;
     }
     const double sr = fma(wr, s1, fma(-n, s2, g.zs[0])), si = wi * s1;
-    coincident = r == 0.0;
-    return fma(r, g.energy_r2, g.energy_0) + log(r * fma(sr, sr, si * si));
+    rest = fma(r, g.energy_r2, g.energy_0);
+    return r * fma(sr, sr, si * si);
 }
 
 // ---------------------------------------------------------------------------------------------
