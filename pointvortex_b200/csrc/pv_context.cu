@@ -105,8 +105,14 @@ struct pv_context {
     DeviceArray pu, pv;              // chunk partials (or symmetric-kernel rows)
     cudaGraphExec_t attempt_graph = nullptr; // one DOPRI5 attempt with a valid FSAL derivative
     SymmetricPlan sym{};             // one evaluation per unordered pair (when planned)
-    DeviceArray sym_items, sym_counter;
-    int sym_items_blocks = 0;        // the block count the item table was built for
+    struct PairItems {               // block pairs of the symmetric form, and their work queue
+        DeviceArray list, counter;
+        int blocks = 0;              // the block count the list was built for
+        const unsigned *items() const { return reinterpret_cast<const unsigned *>(list.p); }
+        unsigned *queue() const { return reinterpret_cast<unsigned *>(counter.p); }
+    };
+    PairItems sym_items;             // the device state's
+    PairItems eval_items;            // host evaluations'
     DeviceArray inv_scratch, inv_out;
     DeviceArray cand;                // dipole candidates (3 doubles-worth each)
     char *stage = nullptr;           // pinned staging, its size, and whether uploads may still read it
@@ -169,7 +175,8 @@ struct pv_context {
         for (DeviceArray *a : {&x, &y, &gamma, &gs, &p0x, &p0y, &p1x, &p1y, &pu, &pv, &inv_scratch,
                                &inv_out, &cand, &ex, &ey, &eg, &egs, &eu, &ev, &epu, &epv,
                                &removed_index, &fmt_stage, &fmt_block, &fmt_out,
-                               &sym_items, &sym_counter, &near_count, &near_slot})
+                               &sym_items.list, &sym_items.counter,
+                               &eval_items.list, &eval_items.counter, &near_count, &near_slot})
             a->release();
         for (int s = 0; s < 7; ++s) {
             kx[s].release();
@@ -575,9 +582,7 @@ pv_status launch_eval(pv_context *c, const double *px, const double *py) {
     if (c->sym.enabled()) {
         PV_CUDA(c, counted(c, PV_KERNEL_VELOCITY, 1, [&] {
                     return launch_symmetric(
-                        px, py, c->gs.p, c->n, c->sym,
-                        reinterpret_cast<const unsigned *>(c->sym_items.p),
-                        reinterpret_cast<unsigned *>(c->sym_counter.p),
+                        px, py, c->gs.p, c->n, c->sym, c->sym_items.items(), c->sym_items.queue(),
                         reinterpret_cast<double2 *>(c->pu.p), padded(c->n), c->gc, lists,
                         c->stream);
                 }));
@@ -675,8 +680,8 @@ std::vector<const void *> attempt_key(const pv_context *c) {
                                    reinterpret_cast<const void *>(
                                        static_cast<uintptr_t>(c->sym.blocks)),
                                    c->x.p, c->y.p, c->gamma.p, c->gs.p, c->p0x.p, c->p0y.p,
-                                   c->p1x.p, c->p1y.p, c->pu.p, c->pv.p, c->sym_items.p,
-                                   c->sym_counter.p, c->ctl, c->cand.p,
+                                   c->p1x.p, c->p1y.p, c->pu.p, c->pv.p, c->sym_items.list.p,
+                                   c->sym_items.counter.p, c->ctl, c->cand.p,
                                    reinterpret_cast<const void *>(static_cast<uintptr_t>(
                                        c->dipole_configured && c->dipole.removal ? 1 : 0)),
                                    reinterpret_cast<const void *>(
@@ -693,6 +698,24 @@ std::vector<const void *> attempt_key(const pv_context *c) {
         k.push_back(c->ky[s].p);
     }
     return k;
+}
+
+cudaError_t ensure_pair_items(pv_context *c, pv_context::PairItems &t, const SymmetricPlan &plan) {
+    if (t.blocks == plan.blocks)
+        return cudaSuccess;
+    t.blocks = 0;
+    std::vector<unsigned> items(plan.items);
+    symmetric_items(plan, items.data());
+    cudaError_t e;
+    if ((e = t.list.ensure((items.size() + 1) / 2)) != cudaSuccess ||
+        (e = t.counter.ensure(1)) != cudaSuccess ||
+        (e = cudaMemsetAsync(t.counter.p, 0, 2 * sizeof(unsigned), c->stream)) != cudaSuccess ||
+        (e = cudaMemcpyAsync(t.list.p, items.data(), items.size() * sizeof(unsigned),
+                             cudaMemcpyHostToDevice, c->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(c->stream)) != cudaSuccess)
+        return e;
+    t.blocks = plan.blocks;
+    return cudaSuccess;
 }
 
 pv_status ensure_state_capacity(pv_context *c, size_t n) {
@@ -718,17 +741,8 @@ pv_status ensure_state_capacity(pv_context *c, size_t n) {
     // the symmetric kernels' rows hold (u, v) pairs in pu's room; the chunk partials use both
     PV_CUDA(c, c->pu.ensure(c->sym.enabled() ? 2 * partial : partial));
     PV_CUDA(c, c->pv.ensure(c->sym.enabled() ? 1 : partial));
-    if (c->sym.enabled() && c->sym_items_blocks != c->sym.blocks) {
-        std::vector<unsigned> items(c->sym.items);
-        symmetric_items(c->sym, items.data());
-        PV_CUDA(c, c->sym_items.ensure((items.size() + 1) / 2));
-        PV_CUDA(c, c->sym_counter.ensure(1));
-        PV_CUDA(c, cudaMemsetAsync(c->sym_counter.p, 0, 2 * sizeof(unsigned), c->stream));
-        PV_CUDA(c, cudaMemcpyAsync(c->sym_items.p, items.data(), items.size() * sizeof(unsigned),
-                                   cudaMemcpyHostToDevice, c->stream));
-        PV_CUDA(c, cudaStreamSynchronize(c->stream));
-        c->sym_items_blocks = c->sym.blocks;
-    }
+    if (c->sym.enabled())
+        PV_CUDA(c, ensure_pair_items(c, c->sym_items, c->sym));
     return PV_OK;
 }
 
@@ -760,8 +774,23 @@ pv_status evaluate_host(pv_context *c, const double *x, const double *y, const d
     PV_CUDA(c, c->ev.ensure(padded(nt)));
     const EvalPlan plan = plan_evaluation(c->gc, nt, n, c->sm_count, 0, c->params.precision);
     const size_t stride = padded(nt);
-    PV_CUDA(c, c->epu.ensure(static_cast<size_t>(plan.num_chunks) * stride));
-    PV_CUDA(c, c->epv.ensure(static_cast<size_t>(plan.num_chunks) * stride));
+    // All targets in FP64: once per unordered pair where the device state would be, since a state's
+    // upload and first evaluation differ from this in nothing (whole calls, ordered and so: box N = 2048
+    // 107 and 93 us, 12 000 657 and 398; disk 4096 114 and 112, 12 000 422 and 300; plane 16 400 373 and
+    // 341, 24 000 623 and 498). Rows that do
+    // not fit into the memory left, which the chunks' partials may, leave the ordered form.
+    SymmetricPlan sym{};
+    if (nt == n && c->params.precision == PV_PRECISION_FP64)
+        sym = plan_symmetric(n, c->sm_count, c->params.precision, c->gc);
+    if (sym.enabled() && (c->epu.ensure(2 * static_cast<size_t>(sym.blocks) * stride) != cudaSuccess ||
+                          ensure_pair_items(c, c->eval_items, sym) != cudaSuccess)) {
+        cudaGetLastError();
+        sym = SymmetricPlan{};
+    }
+    if (!sym.enabled()) {
+        PV_CUDA(c, c->epu.ensure(static_cast<size_t>(plan.num_chunks) * stride));
+        PV_CUDA(c, c->epv.ensure(static_cast<size_t>(plan.num_chunks) * stride));
+    }
     const std::vector<double> gs = scaled(c->gc, g, n);
     {
         const double *src[4] = {x, y, g, gs.data()};
@@ -797,6 +826,11 @@ pv_status evaluate_host(pv_context *c, const double *x, const double *y, const d
         a.near = near_lists(c);
     }
     PV_CUDA(c, counted(c, PV_KERNEL_VELOCITY, 1, [&] {
+                if (sym.enabled())
+                    return launch_symmetric(c->ex.p, c->ey.p, c->egs.p, n, sym, c->eval_items.items(),
+                                            c->eval_items.queue(),
+                                            reinterpret_cast<double2 *>(c->epu.p), stride, a.g,
+                                            f32::NearLists{nullptr, nullptr}, c->stream);
                 return c->params.precision == PV_PRECISION_FP32C
                            ? launch_velocity_fp32c(a, plan, c->stream)
                            : launch_velocity(a, plan, c->stream);
@@ -821,10 +855,14 @@ pv_status evaluate_host(pv_context *c, const double *x, const double *y, const d
     s.n = nt;
     s.mode = STAGE_REDUCE_ONLY;
     s.reduce = 1;
-    s.num_chunks = plan.num_chunks;
+    s.num_chunks = sym.enabled() ? sym.blocks : plan.num_chunks;
     s.stride = stride;
-    s.pu = c->epu.p;
-    s.pv = c->epv.p;
+    if (sym.enabled()) {
+        s.pr = reinterpret_cast<const double2 *>(c->epu.p);
+    } else {
+        s.pu = c->epu.p;
+        s.pv = c->epv.p;
+    }
     s.s = 0;
     s.kx[0] = c->eu.p;
     s.ky[0] = c->ev.p;
