@@ -90,7 +90,8 @@ struct SymmetricPlan {
 constexpr size_t kSymmetricMinN = 2048;       // periodic box below: the ordered kernel
 constexpr size_t kSymmetricPlaneMinN = 16384;   // infinite plane below: the ordered kernel
 constexpr size_t kSymmetricPlane32MinN = 16384; // the same for the FP32-compensated plane
-constexpr size_t kSymmetricPlaneWideN = 32768;  // the plane from here: 8 targets per lane
+constexpr size_t kSymmetricPlaneWideN = 32768;  // the plane from here: 8 targets per lane (16 400: 166 us
+                                                // an evaluation with 4 and 210 with 8; 40 000: 816 and 791)
 // FP64 disk below: the ordered kernel (18 us at 2048; the once-per-pair tiles 19, 36 against 43 at
 // 4096, where 128 blocks of 32 first give every SM work)
 constexpr size_t kSymmetricDiskMinN = 4096;
