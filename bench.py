@@ -42,23 +42,16 @@ WORKLOAD = "periodic_dopri5_n4096"
 L2_BYTES = 126 * 1024 * 1024
 METRIC = "pair-interactions/s"
 
-# Algorithmic FP64 operations per ordered pair of the periodic evaluation (FMA = 2, add/mul/
-# reciprocal/rint = 1), as the truncated image series is evaluated (pv_geometry.cuh,
-# PeriodicPair): per axis the displacement, exact remainder and scaling (7) and the shared
-# sinh/cosh/sin/cos Taylor series of the half angle (48); the derived cosh, cos, sin, sinh of the
-# full angles (20) and the two m = 0 denominators (8); per axis the image sum -- setup (6), the
-# exact m = +-1, +-2 pairs (18), the m = 3..5 expansion (6) and the m = +-6 terms (5); per axis
-# the combination, reciprocal and update (16).
-FLOPS_PER_PAIR_PERIODIC = 240
-# The symmetric form evaluates each unordered pair once and applies it to both vortices: the same
-# 240 plus two more FMA updates (the source's reaction) per unordered pair.
-FLOPS_PER_UNORDERED_PAIR_SYMMETRIC = 244
-# The work these counts state is kept fixed, so that the roofline fraction stays comparable as the
-# kernel changes. What the kernel now executes per unordered pair is less (economized series,
-# shared doubled values, the m = 1, 2 fraction started from m = 1, the m = +-6 images in the
-# m = 3..6 expansion): 189, counted by ncu as 2 x DFMA + DMUL + DADD per unordered pair (72.5,
-# 36.3 and 8.1 FP64 instructions) at N = 4096.
-FLOPS_EXECUTED_PER_UNORDERED_PAIR_SYMMETRIC = 189
+# Algorithmic FP64 operations per pair of the periodic evaluation from six image layers up (FMA = 2,
+# add/mul/reciprocal = 1), as ZetaPair evaluates it (pv_geometry.cuh): z^2, |z|^2, z^4 and its square
+# 12; the two polynomials of the rational function 28; z Q, its square and the reciprocal 16; the two
+# kernel values 12. An ordered pair adds the displacement and its reduction 12 and two FMA updates 4;
+# an unordered one displacement and reduction 4 and four FMA updates 8.
+FLOPS_PER_PAIR_PERIODIC = 84
+FLOPS_PER_UNORDERED_PAIR_SYMMETRIC = 80
+# It executes them in 50 FP64 instructions, 29 of them FMAs (ncu: 50.3 a pair at N = 16 384 with the
+# diagonal items).
+FP64_INSTRUCTIONS_PER_UNORDERED_PAIR = 50
 # The plane in the same count: an ordered pair is 11 (displacement 2, r^2 3, reciprocal 1, scale
 # 1, two FMA updates 4); the symmetric form spends 16 per unordered pair (the shared displacement,
 # r^2 and reciprocal, the two kernel values 2, four FMA updates 8).
@@ -250,10 +243,10 @@ def run_ours(args):
     plan = k.statePlan()
     if plan["symmetric"]:
         flops_per_ordered_pair = FLOPS_PER_UNORDERED_PAIR_SYMMETRIC / 2.0
-        kernel_name = "symmetric_kernel<PeriodicSym, 1>"
+        kernel_name = "symmetric_kernel<ZetaSym, 1>"
     else:
         flops_per_ordered_pair = FLOPS_PER_PAIR_PERIODIC
-        kernel_name = "velocity_kernel<PeriodicPair>"
+        kernel_name = "velocity_kernel<ZetaPair>"
     achieved = flops_per_ordered_pair * pairs_profiled / (v_ms * 1e-3) / 1e12
     # measured FP64 FMA peak of this GPU (36.8 TFLOP/s at 1965 MHz on this pool's B200s when
     # the probe is skipped, e.g. under a profiler)
@@ -290,15 +283,16 @@ def run_ours(args):
                          "kernel": kernel_name,
                          "flops_per_pair": flops_per_ordered_pair,
                          "flops_executed_per_pair": (
-                             FLOPS_EXECUTED_PER_UNORDERED_PAIR_SYMMETRIC / 2.0
+                             FLOPS_PER_UNORDERED_PAIR_SYMMETRIC / 2.0
                              if plan["symmetric"] else None),
-                         "flops_note": "FP64 operations per ordered pair as the periodic series "
-                                       "was first evaluated (FMA = 2), the implementation's own "
-                                       "tally rather than a formula minimum, so frac reads as "
-                                       "FP64-pipe work; kept fixed across kernel changes (the "
-                                       "kernel now executes flops_executed_per_pair). "
-                                       "Per ordered pair of the launched "
-                                       "kernel (the symmetric form: 244 per unordered pair)",
+                         "fp64_instructions_per_unordered_pair": (
+                             FP64_INSTRUCTIONS_PER_UNORDERED_PAIR if plan["symmetric"] else None),
+                         "flops_note": "FP64 operations per ordered pair as the rational box term "
+                                       "evaluates it (FMA = 2), the implementation's own tally "
+                                       "rather than a formula minimum (the symmetric form: 80 per "
+                                       "unordered pair, 50 instructions, of which 29 are FMAs: all "
+                                       "of the FP64 pipe's issue slots would read 0.8 of the FMA "
+                                       "peak)",
                          "ms_per_launch": per_launch_ms, "launches": v_timed,
                          "timing": "CUDA events around each launch on the library stream, in a "
                                    "second pass of the same number of steps right after the "
