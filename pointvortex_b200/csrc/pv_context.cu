@@ -1202,6 +1202,9 @@ pv_status enqueue_small_steps(pv_context *c, SmallSteps &p) {
     p.k0y = c->ky[0].p;
     p.ctl = c->ctl;
     p.spin_limit = c->spin_limit;
+    // a context with a limit of its own keeps the barrier that has one
+    p.cluster = c->spin_limit == kGridSpinLimit &&
+                small_steps_in_cluster(c->gc, c->n, c->plan.num_chunks);
     p.g = c->gc;
     PV_CUDA(c, counted(c, PV_KERNEL_VELOCITY, 1,
                        [&] { return launch_small_steps(p, c->sm_count, c->stream); }));

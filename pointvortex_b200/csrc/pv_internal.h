@@ -200,11 +200,13 @@ struct SmallSteps {
     uint64_t steps;
     double dt;
     DeviceControl *ctl;
+    int cluster;            // one cluster instead of the whole grid
     uint32_t spin_limit = kGridSpinLimit;  // polls of a grid-barrier wait (pv_set_wait_limits)
     GeometryConsts g;
 };
 constexpr size_t kSmallStepsMaxN = 2048;
 bool small_steps_eligible(size_t n, int num_chunks, int sm_count);
+bool small_steps_in_cluster(const GeometryConsts &g, size_t n, int num_chunks);
 cudaError_t launch_small_steps(const SmallSteps &p, int sm_count, cudaStream_t stream);
 
 // Accept kernel: state <- xt (and, for DOPRI5, k0 <- k6 when the attempt was accepted).

@@ -583,6 +583,10 @@ struct GridBarrier {
     unsigned long long open_at;  // of the next barrier
     unsigned parity;
 
+    __device__ __forceinline__ explicit GridBarrier(const SmallSteps &p)
+        : arrivals(&p.ctl->arrivals), status(&p.ctl->status), limit(p.spin_limit), open_at(0ull),
+          parity(0u) {}
+
     // Returns true when the barrier opened and no CTA arrived with an error. bad: this thread met one.
     __device__ __forceinline__ bool wait(bool bad) {
         __shared__ int go;
@@ -633,6 +637,50 @@ struct GridBarrier {
     }
 };
 
+// The same steps in one cluster of kClusterSteps CTAs, for populations whose pairs so few SMs evaluate
+// as fast as the grid exchanges positions: the barrier is the hardware's, and each stage's positions go
+// straight into the other buffer of every CTA's shared memory, where the next evaluation reads them. A
+// CTA that met an error tells every CTA through a flag there, by the barrier's parity as above. The
+// hardware's barrier has no limit to set; it cannot stay shut, since a cluster's CTAs are resident
+// together and each takes the same way through the phases. A stage saves about 1 us: RK4 steps at
+// N = 128, grid and cluster: plane 12.1 and 8.2 us, disk 14.1 and 10.1, box 18.2 and 14.2.
+constexpr unsigned kClusterSteps = 16;
+
+__device__ __forceinline__ uint32_t remote_shared(const void *local, unsigned rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(a)
+        : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(local))), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+struct ClusterBarrier {
+    int *flags;  // [2] in this CTA's shared memory
+    unsigned parity;
+
+    __device__ __forceinline__ explicit ClusterBarrier(const SmallSteps &) : parity(0u) {
+        __shared__ int shared_flags[2];
+        flags = shared_flags;
+        if (threadIdx.x < 2)
+            flags[threadIdx.x] = 0;
+    }
+    __device__ __forceinline__ bool wait(bool bad) {
+        parity ^= 1u;
+        if (bad)
+            for (unsigned rank = 0; rank < kClusterSteps; ++rank)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(
+                                 remote_shared(flags + parity, rank)),
+                             "r"(1)
+                             : "memory");
+        cluster_sync();
+        return *static_cast<volatile int *>(flags + parity) == 0;
+    }
+};
+
 // Sources whose pair chains overlap in a thread's chunk sum.
 template <class Pair> struct ChunkUnroll { static constexpr int value = 4; };
 template <> struct ChunkUnroll<InfinitePair> { static constexpr int value = 16; };
@@ -642,8 +690,9 @@ constexpr int kStepThreads = 256;
 
 // Shared memory of a CTA: all sources, its targets' chunk sums, and per target what its finish
 // keeps from stage to stage.
-struct StepShared {
+template <bool CLUSTER> struct StepShared {
     double *x, *y, *g;    // [n]
+    double *xn, *yn;      // [n]: a cluster's next positions
     double *qu, *qv;      // [targets][chunks]
     double *k;            // [7][2][targets]: stage velocities
     double *x0, *y0;      // [targets]: the step's start
@@ -657,32 +706,75 @@ struct StepShared {
         k = qv + targets * chunks;
         x0 = k + 14 * targets;
         y0 = x0 + targets;
+        xn = y0 + targets;
+        yn = xn + np;
+    }
+    // Position of target i for the next evaluation: to every CTA, or to the exchange's buffer `to`.
+    __device__ __forceinline__ void publish(const SmallSteps &p, int to, size_t i, double px,
+                                            double py) const {
+        if (CLUSTER) {
+#pragma unroll 4
+            for (unsigned rank = 0; rank < kClusterSteps; ++rank) {
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote_shared(xn + i, rank)),
+                             "d"(px)
+                             : "memory");
+                asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote_shared(yn + i, rank)),
+                             "d"(py)
+                             : "memory");
+            }
+        } else {
+            p.px[to][i] = px;
+            p.py[to][i] = py;
+        }
+    }
+    // After the barrier that follows publish().
+    __device__ __forceinline__ void turn() {
+        if (CLUSTER) {
+            double *t = x;
+            x = xn;
+            xn = t;
+            t = y;
+            y = yn;
+            yn = t;
+        }
+    }
+    // A cluster's first positions, and every CTA started before any writes into another's memory.
+    __device__ __forceinline__ void begin(const SmallSteps &p) const {
+        if (CLUSTER) {
+            for (size_t j = threadIdx.x; j < p.n; j += kStepThreads) {
+                x[j] = p.x[j];
+                y[j] = p.y[j];
+            }
+            cluster_sync();
+        }
     }
 };
-size_t step_shared_bytes(size_t n, size_t targets, int chunks) {
+size_t step_shared_bytes(size_t n, size_t targets, int chunks, bool cluster) {
     const size_t np = (n + 1) & ~static_cast<size_t>(1);
-    return (3 * np + 2 * targets * static_cast<size_t>(chunks) + 16 * targets) * sizeof(double);
+    return ((cluster ? 5 : 3) * np + 2 * targets * static_cast<size_t>(chunks) + 16 * targets) * sizeof(double);
 }
 
-// One evaluation: positions (px, py) into shared memory, then the chunk sums of the CTA's targets
-// [t0, t0 + mine).
-template <class Pair>
-__device__ __forceinline__ void step_evaluate(const SmallSteps &p, const StepShared &sh,
+// One evaluation: positions (px, py) into shared memory (a cluster's are there), then the chunk sums of
+// the CTA's targets [t0, t0 + mine).
+template <class Pair, bool CLUSTER>
+__device__ __forceinline__ void step_evaluate(const SmallSteps &p, const StepShared<CLUSTER> &sh,
                                               const double *px, const double *py, size_t t0,
                                               int mine) {
-    const int n2 = static_cast<int>(p.n / 2);
-    const double2 *px2 = reinterpret_cast<const double2 *>(px);
-    const double2 *py2 = reinterpret_cast<const double2 *>(py);
+    if (!CLUSTER) {
+        const int n2 = static_cast<int>(p.n / 2);
+        const double2 *px2 = reinterpret_cast<const double2 *>(px);
+        const double2 *py2 = reinterpret_cast<const double2 *>(py);
 #pragma unroll 4  // the loads of several iterations in flight at once
-    for (int j = threadIdx.x; j < n2; j += kStepThreads) {
-        reinterpret_cast<double2 *>(sh.x)[j] = __ldcg(px2 + j);
-        reinterpret_cast<double2 *>(sh.y)[j] = __ldcg(py2 + j);
+        for (int j = threadIdx.x; j < n2; j += kStepThreads) {
+            reinterpret_cast<double2 *>(sh.x)[j] = __ldcg(px2 + j);
+            reinterpret_cast<double2 *>(sh.y)[j] = __ldcg(py2 + j);
+        }
+        if ((p.n & 1) && threadIdx.x == 0) {
+            sh.x[p.n - 1] = __ldcg(px + p.n - 1);
+            sh.y[p.n - 1] = __ldcg(py + p.n - 1);
+        }
+        __syncthreads();
     }
-    if ((p.n & 1) && threadIdx.x == 0) {
-        sh.x[p.n - 1] = __ldcg(px + p.n - 1);
-        sh.y[p.n - 1] = __ldcg(py + p.n - 1);
-    }
-    __syncthreads();
     const int nc = p.num_chunks;
     for (int w = threadIdx.x; w < mine * nc; w += kStepThreads) {
         const int li = w % mine, c = w / mine;
@@ -711,8 +803,9 @@ __device__ __forceinline__ void step_evaluate(const SmallSteps &p, const StepSha
 
 // The velocity of target li from its chunk sums (the slow path included), kept as stage s's. Returns
 // an error status, or 0.
-__device__ __forceinline__ int step_velocity(const SmallSteps &p, const StepShared &sh, int li,
-                                             size_t i, int targets, int s) {
+template <bool CLUSTER>
+__device__ __forceinline__ int step_velocity(const SmallSteps &p, const StepShared<CLUSTER> &sh,
+                                             int li, size_t i, int targets, int s) {
     double ku, kv;
     const double *qu = sh.qu + li * p.num_chunks, *qv = sh.qv + li * p.num_chunks;
     sum_chunks(
@@ -731,8 +824,9 @@ __device__ __forceinline__ int step_velocity(const SmallSteps &p, const StepShar
 }
 
 // Stage position x0 + dt sum_j a_j k_j of component `part` (makeStage, src/timestep.cpp:19-30).
-__device__ __forceinline__ double step_position(const StepShared &sh, const double *row, int ncoef,
-                                                int part, int li, int targets, double x0,
+template <bool CLUSTER>
+__device__ __forceinline__ double step_position(const StepShared<CLUSTER> &sh, const double *row,
+                                                int ncoef, int part, int li, int targets, double x0,
                                                 double dt) {
     double d = 0.0;
     for (int j = 0; j < ncoef; ++j)
@@ -741,16 +835,17 @@ __device__ __forceinline__ double step_position(const StepShared &sh, const doub
     return __dadd_rn(x0, __dmul_rn(dt, d));
 }
 
-template <class Pair>
+template <class Pair, bool CLUSTER>
 __global__ void __launch_bounds__(kStepThreads, 1) rk4_steps_kernel(const SmallSteps p) {
     extern __shared__ __align__(16) double smem[];
     const int targets = static_cast<int>((p.n + gridDim.x - 1) / gridDim.x);
     const size_t t0 = static_cast<size_t>(blockIdx.x) * targets;
     const int mine = t0 < p.n ? static_cast<int>(min(static_cast<size_t>(targets), p.n - t0)) : 0;
-    const StepShared sh(smem, p.n, targets, p.num_chunks);
+    StepShared<CLUSTER> sh(smem, p.n, targets, p.num_chunks);
     for (size_t j = threadIdx.x; j < p.n; j += kStepThreads)
         sh.g[j] = p.gs[j];
-    GridBarrier barrier{&p.ctl->arrivals, &p.ctl->status, p.spin_limit, 0ull, 0u};
+    std::conditional_t<CLUSTER, ClusterBarrier, GridBarrier> barrier(p);
+    sh.begin(p);
     const int li = threadIdx.x;  // a target's finish is its own thread's
     const size_t i = t0 + li;
     for (uint64_t step = 0; step < p.steps; ++step) {
@@ -759,7 +854,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) rk4_steps_kernel(const SmallS
             // previous step's combination (not yet copied into the state); then the last stage's
             const double *px = s == 0 ? (step > 0 ? p.px[1] : p.x) : p.px[(s - 1) & 1];
             const double *py = s == 0 ? (step > 0 ? p.py[1] : p.y) : p.py[(s - 1) & 1];
-            step_evaluate<Pair>(p, sh, px, py, t0, mine);
+            step_evaluate<Pair, CLUSTER>(p, sh, px, py, t0, mine);
             int error = 0;
             if (li < mine) {
                 if (s == 0) {
@@ -785,35 +880,36 @@ __global__ void __launch_bounds__(kStepThreads, 1) rk4_steps_kernel(const SmallS
                     if (!isfinite(nx) || !isfinite(ny))
                         error = max(error, static_cast<int>(ST_NONFINITE_POSITION));
                 }
-                p.px[s & 1][i] = nx;
-                p.py[s & 1][i] = ny;
+                sh.publish(p, s & 1, i, nx, ny);
                 if (error)
                     set_status(&p.ctl->status, error);
             }
             if (!barrier.wait(error != 0))
                 return;
+            sh.turn();
         }
     }
     if (li < mine) {  // the last step's accept
-        p.x[i] = __ldcg(p.px[1] + i);
-        p.y[i] = __ldcg(p.py[1] + i);
+        p.x[i] = CLUSTER ? sh.x[i] : __ldcg(p.px[1] + i);
+        p.y[i] = CLUSTER ? sh.y[i] : __ldcg(p.py[1] + i);
     }
 }
 
 // One adaptive step (src/timestep.cpp:62-120). need_k0: the derivative at the state is not cached in
 // (k0x, k0y). A rejected attempt changes only the step size, so the next one starts from the same
 // k0 without leaving the kernel; an accepted one updates the state and k0.
-template <class Pair>
+template <class Pair, bool CLUSTER>
 __global__ void __launch_bounds__(kStepThreads, 1) dopri_step_kernel(const SmallSteps p) {
     extern __shared__ __align__(16) double smem[];
     __shared__ double s_error;
     const int targets = static_cast<int>((p.n + gridDim.x - 1) / gridDim.x);
     const size_t t0 = static_cast<size_t>(blockIdx.x) * targets;
     const int mine = t0 < p.n ? static_cast<int>(min(static_cast<size_t>(targets), p.n - t0)) : 0;
-    const StepShared sh(smem, p.n, targets, p.num_chunks);
+    StepShared<CLUSTER> sh(smem, p.n, targets, p.num_chunks);
     for (size_t j = threadIdx.x; j < p.n; j += kStepThreads)
         sh.g[j] = p.gs[j];
-    GridBarrier barrier{&p.ctl->arrivals, &p.ctl->status, p.spin_limit, 0ull, 0u};
+    std::conditional_t<CLUSTER, ClusterBarrier, GridBarrier> barrier(p);
+    sh.begin(p);
     const int li = threadIdx.x;
     const size_t i = t0 + li;
     const bool owner = li < mine;
@@ -838,8 +934,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) dopri_step_kernel(const Small
         for (int s = 0; s < 7; ++s) {
             const bool evaluate = s > 0 || (p.need_k0 && attempt == 0);
             if (evaluate)
-                step_evaluate<Pair>(p, sh, s == 0 ? p.x : p.px[(s - 1) & 1],
-                                    s == 0 ? p.y : p.py[(s - 1) & 1], t0, mine);
+                step_evaluate<Pair, CLUSTER>(p, sh, s == 0 ? p.x : p.px[(s - 1) & 1],
+                                             s == 0 ? p.y : p.py[(s - 1) & 1], t0, mine);
             int error = 0;
             if (owner) {
                 if (evaluate)
@@ -847,8 +943,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) dopri_step_kernel(const Small
                 if (s < 6) {
                     x5 = step_position(sh, p.rows[s + 1], s + 1, 0, li, targets, sh.x0[li], dt);
                     y5 = step_position(sh, p.rows[s + 1], s + 1, 1, li, targets, sh.y0[li], dt);
-                    p.px[s & 1][i] = x5;
-                    p.py[s & 1][i] = y5;
+                    sh.publish(p, s & 1, i, x5, y5);
                     error = max(error, position_error(p.g, x5, y5));
                 } else {  // (x5, y5): the fifth-order point, the position of k6
                     double xe = 0.0, ye = 0.0;
@@ -881,6 +976,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) dopri_step_kernel(const Small
                     ctl->attempts = attempt + 1;
                 return;
             }
+            if (s < 6)
+                sh.turn();
         }
         if (threadIdx.x == 0)
             s_error = __longlong_as_double(
@@ -913,6 +1010,15 @@ __global__ void __launch_bounds__(kStepThreads, 1) dopri_step_kernel(const Small
     }
 }
 
+// While a CTA of the cluster has a thread for each (target, chunk); the box, whose pairs take five times
+// the plane's FP64 cycles, while it has two. Measured at both sides (us an RK4 step, cluster and grid):
+// plane N = 300 11.4 and 14.1, 400 17.8 and 13.4; disk 300 14.8 and 15.4, 400 23.8 and 14.6; box 200
+// 14.8 and 18.4, 256 20.9 and 18.5.
+bool small_steps_in_cluster(const GeometryConsts &g, size_t n, int num_chunks) {
+    const size_t units = (n + kClusterSteps - 1) / kClusterSteps * static_cast<size_t>(num_chunks);
+    return units <= (g.geometry == GEO_PERIODIC ? kStepThreads / 2 : kStepThreads);
+}
+
 bool small_steps_eligible(size_t n, int num_chunks, int sm_count) {
     const size_t grid = static_cast<size_t>(sm_count > 0 ? sm_count : 148);
     return n >= 1 && n <= kSmallStepsMaxN && num_chunks >= 1 && num_chunks < kWideRows &&
@@ -920,14 +1026,15 @@ bool small_steps_eligible(size_t n, int num_chunks, int sm_count) {
 }
 
 namespace {
+// The whole grid, one CTA per SM, cooperative (every CTA resident, or no launch at all), or one cluster.
 template <class Kernel>
-cudaError_t launch_cooperative(Kernel kernel, const SmallSteps &p, int sm_count,
-                               cudaStream_t stream) {
-    const size_t grid =
-        std::min<size_t>(static_cast<size_t>(sm_count > 0 ? sm_count : 148), p.n);
-    const size_t smem = step_shared_bytes(p.n, (p.n + grid - 1) / grid, p.num_chunks);
+cudaError_t launch_steps(Kernel kernel, const SmallSteps &p, size_t grid, bool cluster,
+                         cudaStream_t stream) {
+    const size_t smem = step_shared_bytes(p.n, (p.n + grid - 1) / grid, p.num_chunks, cluster);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(smem));
+    if (e == cudaSuccess && cluster)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess)
         return e;
     cudaLaunchConfig_t cfg = {};
@@ -936,8 +1043,14 @@ cudaError_t launch_cooperative(Kernel kernel, const SmallSteps &p, int sm_count,
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;  // every CTA resident, or no launch at all
-    attr[0].val.cooperative = 1;
+    if (cluster) {
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = kClusterSteps;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    } else {
+        attr[0].id = cudaLaunchAttributeCooperative;
+        attr[0].val.cooperative = 1;
+    }
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, p);
@@ -945,8 +1058,18 @@ cudaError_t launch_cooperative(Kernel kernel, const SmallSteps &p, int sm_count,
 
 template <class Pair>
 cudaError_t launch_small(const SmallSteps &p, int sm_count, cudaStream_t stream) {
-    return p.dopri ? launch_cooperative(dopri_step_kernel<Pair>, p, sm_count, stream)
-                   : launch_cooperative(rk4_steps_kernel<Pair>, p, sm_count, stream);
+    if (p.cluster) {
+        const cudaError_t e =
+            p.dopri ? launch_steps(dopri_step_kernel<Pair, true>, p, kClusterSteps, true, stream)
+                    : launch_steps(rk4_steps_kernel<Pair, true>, p, kClusterSteps, true, stream);
+        if (e == cudaSuccess)
+            return e;
+        cudaGetLastError();  // no GPC with that many SMs free for a cluster: the grid
+    }
+    const size_t grid =
+        std::min<size_t>(static_cast<size_t>(sm_count > 0 ? sm_count : 148), p.n);
+    return p.dopri ? launch_steps(dopri_step_kernel<Pair, false>, p, grid, false, stream)
+                   : launch_steps(rk4_steps_kernel<Pair, false>, p, grid, false, stream);
 }
 } // namespace
 
