@@ -18,6 +18,11 @@ namespace pvb {
 namespace {
 constexpr int kHT = 128;                // Hamiltonian tile edge (threads per block)
 constexpr int kMomentBlocks = 256;
+// Small populations: four (two) blocks share a tile's sources up to 16 (32) tiles an edge, where a
+// thread's 128 pairs one after another are the kernel's time (N = 256 to 2048: 16.6 us, with 32 pairs a
+// thread 7.5; whole calls, box, plane and disk: N = 1024 61, 56 and 58 us, so 45, 44 and 45; N = 3000 69,
+// 57 and 63, so 69, 53 and 57). Returned as a shift.
+unsigned tile_split(size_t nt) { return nt <= 16 ? 2 : (nt <= 32 ? 1 : 0); }
 
 // Neumaier's improvement of Kahan summation: s + c carries the sum with the rounding error of
 // every addition accumulated in c.
@@ -192,9 +197,9 @@ __device__ __forceinline__ bool regular_pairs(const GeometryConsts &gc, double x
 template <int GEO, bool ZETA = false>
 __global__ void __launch_bounds__(kHT)
     hamiltonian_kernel(const double *x, const double *y, const double *g, size_t n,
-                       GeometryConsts gc, double *part, int *status) {
+                       GeometryConsts gc, unsigned split, double *part, int *status) {
     pdl_enter();
-    const unsigned tile_index = blockIdx.x;
+    const unsigned tile_index = blockIdx.x >> split, share = blockIdx.x & ((1u << split) - 1);
     unsigned J = static_cast<unsigned>((sqrt(8.0 * tile_index + 1.0) - 1.0) * 0.5);
     while (static_cast<unsigned long long>(J + 1) * (J + 2) / 2 <= tile_index)
         ++J;
@@ -225,8 +230,9 @@ __global__ void __launch_bounds__(kHT)
         __syncthreads();
     if (i < n) {
         gi = g[i];
-        const int jcount = static_cast<int>(min(static_cast<size_t>(kHT), n - j0));
-        const int jstart = (I == J) ? static_cast<int>(threadIdx.x) + 1 : 0;
+        const int sources = kHT >> split, first = static_cast<int>(share) * sources;
+        const int jcount = static_cast<int>(min(static_cast<size_t>(first + sources), n - j0));
+        const int jstart = max(first, (I == J) ? static_cast<int>(threadIdx.x) + 1 : 0);
         bool done = false;
         if (kRegular)
             done = near ? regular_pairs<GEO, ZETA, true>(gc, xi, yi, sx, sy, sg, table, jstart, jcount,
@@ -238,7 +244,7 @@ __global__ void __launch_bounds__(kHT)
             for (int jj = jstart; jj < jcount; ++jj)
                 acc.add(sg[jj] * energy<GEO, ZETA>(gc, xi, yi, sx[jj], sy[jj], status));
         }
-        if (GEO == GEO_DISK && I == J) {
+        if (GEO == GEO_DISK && I == J && share == 0) {
             const double ri2 = __dadd_rn(__dmul_rn(xi, xi), __dmul_rn(yi, yi));
             if (ri2 >= gc.radius2)
                 set_status(status, ST_OUTSIDE_DISK_H);
@@ -248,26 +254,32 @@ __global__ void __launch_bounds__(kHT)
     const double hi = block_sum_fixed(gi * acc.s, sh);
     const double lo = block_sum_fixed(gi * acc.c, sh);
     if (threadIdx.x == 0) {
-        part[2 * tile_index] = hi;
-        part[2 * tile_index + 1] = lo;
+        part[2 * blockIdx.x] = hi;
+        part[2 * blockIdx.x + 1] = lo;
     }
 }
 
-// One block: fixed-order compensated sum of the moment partials and Hamiltonian partials.
+// One block: fixed-order compensated sums of the moment partials (a warp each) and of the Hamiltonian
+// partials.
 __global__ void __launch_bounds__(1024)
     finalize_kernel(const double *part, int moment_blocks, size_t tiles, double *out, int *status,
                     int *status_h) {
     pdl_enter();
     __shared__ double sh[32];
-    for (int k = 0; k < 4; ++k) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp < 4) {
         CSum c;
-        for (int b = threadIdx.x; b < moment_blocks; b += blockDim.x)
-            c.add(part[4 * b + k]);
-        const double hi = block_sum_fixed(c.s, sh);
-        const double lo = block_sum_fixed(c.c, sh);
-        if (threadIdx.x == 0) {
-            out[k] = hi + lo;
-            if (!isfinite(out[k]))
+#pragma unroll 8
+        for (int b = lane; b < moment_blocks; b += 32)
+            c.add(part[4 * b + warp]);
+        double hi = c.s, lo = c.c;
+        for (int off = 16; off > 0; off >>= 1) {
+            hi += __shfl_down_sync(0xffffffffu, hi, off);
+            lo += __shfl_down_sync(0xffffffffu, lo, off);
+        }
+        if (lane == 0) {
+            out[warp] = hi + lo;
+            if (!isfinite(hi + lo))
                 set_status_if_clean(status, ST_NONFINITE_MOMENT);
         }
     }
@@ -292,7 +304,8 @@ bool g_tables_ready[64] = {};
 
 size_t invariants_scratch_doubles(size_t n, int) {
     const size_t nt = (n + kHT - 1) / kHT;
-    return 4 * static_cast<size_t>(kMomentBlocks) + 2 * (nt > 0 ? nt * (nt + 1) / 2 : 1);
+    return 4 * static_cast<size_t>(kMomentBlocks) +
+           2 * (nt > 0 ? (nt * (nt + 1) / 2) << tile_split(nt) : 1);
 }
 
 cudaError_t launch_invariants(const double *x, const double *y, const double *gamma, size_t n,
@@ -322,7 +335,8 @@ cudaError_t launch_invariants(const double *x, const double *y, const double *ga
     const size_t nt = (n + kHT - 1) / kHT;
     size_t tiles = 0;
     if (nt > 0) {
-        tiles = nt * (nt + 1) / 2;
+        const unsigned split = tile_split(nt);
+        tiles = (nt * (nt + 1) / 2) << split;
         if (tiles > 0x7fffffffu)
             return cudaErrorInvalidValue;
         const dim3 grid(static_cast<unsigned>(tiles));
@@ -330,17 +344,17 @@ cudaError_t launch_invariants(const double *x, const double *y, const double *ga
         switch (g.geometry) {
         case GEO_INFINITE:
             e = launch_pdl(hamiltonian_kernel<GEO_INFINITE>, grid, dim3(kHT), 0, stream, x, y, gamma,
-                           n, g, hp, status_h);
+                           n, g, split, hp, status_h);
             break;
         case GEO_PERIODIC:
             e = g.zeta ? launch_pdl(hamiltonian_kernel<GEO_PERIODIC, true>, grid, dim3(kHT), 0,
-                                    stream, x, y, gamma, n, g, hp, status_h)
+                                    stream, x, y, gamma, n, g, split, hp, status_h)
                        : launch_pdl(hamiltonian_kernel<GEO_PERIODIC>, grid, dim3(kHT), 0, stream, x,
-                                    y, gamma, n, g, hp, status_h);
+                                    y, gamma, n, g, split, hp, status_h);
             break;
         default:
             e = launch_pdl(hamiltonian_kernel<GEO_DISK>, grid, dim3(kHT), 0, stream, x, y, gamma, n,
-                           g, hp, status_h);
+                           g, split, hp, status_h);
             break;
         }
         if (e != cudaSuccess)

@@ -82,3 +82,11 @@ def test_coincident_pair_in_the_last_tile(kernel):
     x[299], y[299] = x[290], y[290]
     with pytest.raises(RuntimeError, match="coincident"):
         kernel().invariants(VortexSystem(x, y, np.ones(300)))
+
+
+@pytest.mark.parametrize("n", [31, 33, 63, 65, 97, 160, 2047, 2048, 2049, 4096, 4097])
+@pytest.mark.parametrize("radius", [None, 1.0])
+def test_shared_tiles(n, radius):
+    """The shares of a tile's sources that four blocks take up to 2048 vortices
+    and two up to 4096, whole, ragged and empty."""
+    test_tiles(n, radius)
