@@ -78,13 +78,14 @@ int batch_targets_for(int geometry, int precision, size_t n) {
 // a function of the simulation's own geometry, precision and population and of the tables.
 //   * the periodic box from kSymmetricMinN up, both forms, unless its table
 //     (pv_set_symmetric_tuning) says otherwise;
-//   * FP64, the box and the disk from one whole block up to kPairRowsMaxN, where the batch table has
-//     no entry (an entry asks for ordered items). Their pairs cost less than half there (box 50 FP64
-//     instructions against 98 for the two ordered pairs, disk 34 against 58), and the items are a
-//     quarter of an ordered item's (128 x 512), so the queue's last round is fuller. 96 members of
-//     64 to 4096 vortices, geometries in turn: 3.40 ms an attempt with ordered items and
-//     PeriodicPair, 1.88 ms now. The plane's (13 against 20) would be bound by the tile's shuffles
-//     and shared loads;
+//   * FP64, every geometry from one whole block up to kPairRowsMaxN, where the batch table has
+//     no entry (an entry asks for ordered items). Their pairs cost less there (FP64 instructions against
+//     the two ordered pairs': box 50 and 98, disk 32 and 58, plane 13 and 20), and the items are a
+//     quarter of an ordered item's (128 x 512), so the queue's last round is fuller. An attempt of 96
+//     members of 64 to 4096 vortices, geometries in turn: 3.40 ms with ordered items and PeriodicPair,
+//     1.94 ms with one target a lane and the plane ordered, 1.62 ms with four (box: two) and all;
+//     full batches of one size, one target a lane (plane: ordered) and now, us: disk 24 x 4096 3572 and
+//     2998, box 5438 and 5040, plane 1894 and 1508, plane 300 x 256 392 and 338;
 //   * kPairRowsMaxN bounds the partial rows of these smaller members: kPairRows a vortex, which the
 //     arena holds beside the caller's own (pv_batch_create), so no admission is refused for them.
 constexpr size_t kPairRows = 32;
@@ -95,9 +96,10 @@ bool batch_pair_items(const GeometryConsts &g, int precision, size_t n) {
     const int tuned = symmetric_tuning_lookup(g.geometry, precision, n) & 15;
     if (g.geometry == GEO_PERIODIC && (tuned == 2 || (tuned == 0 && n >= kSymmetricMinN)))
         return true;
-    return precision == PV_PRECISION_FP64 && n <= kPairRowsMaxN && tuned == 0 &&
-           (g.geometry == GEO_DISK || (g.geometry == GEO_PERIODIC && g.zeta)) &&
-           batch_entry(g.geometry, precision, n) == 0;
+    if (precision != PV_PRECISION_FP64 || n > kPairRowsMaxN || batch_entry(g.geometry, precision, n) != 0)
+        return false;
+    // the table of single simulations does not speak for the plane, whose rows it judges at their size
+    return g.geometry == GEO_INFINITE || (tuned == 0 && (g.geometry == GEO_DISK || g.zeta));
 }
 // Sources per work item, a function of the population only (so a simulation's summation order
 // never depends on its batch): 512 up to N = 16384, then N/32 rounded up to 512.
@@ -273,12 +275,79 @@ __device__ __forceinline__ void run_item(const GeometryConsts &g, const double *
         }
 }
 
-// One 128 x 128 block pair of an FP64 simulation, once per unordered pair: warp w holds targets
-// I*128 + 32w + lane and meets the four 32-source sub-tiles of block J in turn. Targets' sums go to
-// row J, the sources' reactions (summed over the four warps in fixed order) to row I. A diagonal
-// item (I == J) is evaluated one-sided. red_u / red_v: 4 x 128 doubles of shared memory; src: the
-// warp's source buffer.
-template <class P>
+// A 128 x 128 block pair (I < J), once per unordered pair: warp w holds T targets a lane, of share
+// w % H of block I's H = 4 / T, and meets H of block J's 32-source sub-tiles, from (w / H) H on. The T
+// warps of a share, and the H of a sub-tile, add up in fixed order.
+template <class P, int T, class Load>
+__device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Load &vortex, size_t n,
+                                              unsigned I, unsigned J, double *pu, double *pv,
+                                              size_t pad_n, double *red_u, double *red_v,
+                                              sym::SourceBuffer &src) {
+    constexpr int H = 4 / T;
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, share = w % H, group = w / H;
+    sym::Vortex t[T];
+    bool t_ok[T], all_ok = true, near = true;
+    double u[T], v[T];
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        const size_t ti = static_cast<size_t>(I) * kBlock + (share * T + k) * 32 + lane;
+        t_ok[k] = ti < n;
+        all_ok = all_ok && t_ok[k];
+        t[k] = vortex(ti);
+        near = near && P::near(g, t[k].x, t[k].y);
+        u[k] = v[k] = 0.0;
+    }
+#pragma unroll 1
+    for (int q = H * group; q < H * group + H; ++q) {
+        const size_t sj = static_cast<size_t>(J) * kBlock + static_cast<size_t>(q) * 32 + lane;
+        const int s_ok = sj < n ? 1 : 0;
+        const sym::Vortex s = vortex(sj);
+        double ru = 0.0, rv = 0.0;
+        if (__all_sync(0xffffffffu, all_ok && s_ok)) {
+            sym::react_tiles_full<P, T, true>(g, t, s, src, near, u, v, ru, rv);
+        } else {
+#pragma unroll
+            for (int k = 0; k < T; ++k)
+                sym::react_tile_t<P, false>(g, t[k], t_ok[k], s, s_ok, u[k], v[k], ru, rv);
+        }
+        if (H > 1) {
+            red_u[(T + share) * kBlock + q * 32 + lane] = ru;
+            red_v[(T + share) * kBlock + q * 32 + lane] = rv;
+        } else if (s_ok) {
+            pu[static_cast<size_t>(I) * pad_n + sj] = ru;
+            pv[static_cast<size_t>(I) * pad_n + sj] = rv;
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < T; ++k) {
+        red_u[group * kBlock + (share * T + k) * 32 + lane] = u[k];
+        red_v[group * kBlock + (share * T + k) * 32 + lane] = v[k];
+    }
+    __syncthreads();
+    const auto add = [](const double *red, int rows) {
+        double sum = red[threadIdx.x];
+        for (int k = 1; k < rows; ++k)
+            sum += red[k * kBlock + threadIdx.x];
+        return sum;
+    };
+    const size_t ti = static_cast<size_t>(I) * kBlock + threadIdx.x;
+    const size_t sj = static_cast<size_t>(J) * kBlock + threadIdx.x;
+    if (ti < n) {
+        pu[static_cast<size_t>(J) * pad_n + ti] = add(red_u, T);
+        pv[static_cast<size_t>(J) * pad_n + ti] = add(red_v, T);
+    }
+    if (H > 1 && sj < n) {
+        pu[static_cast<size_t>(I) * pad_n + sj] = add(red_u + T * kBlock, H);
+        pv[static_cast<size_t>(I) * pad_n + sj] = add(red_v + T * kBlock, H);
+    }
+    __syncthreads();
+}
+
+// One 128 x 128 block pair of an FP64 simulation, once per unordered pair by run_pair_item(). Targets'
+// sums go to row J, the sources' reactions to row I. A diagonal item (I == J) is evaluated one-sided:
+// warp w holds targets I*128 + 32w + lane and meets the four 32-source sub-tiles in turn. red_u / red_v:
+// 4 x 128 doubles of shared memory; src: the warp's source buffer.
+template <class P, int T>
 __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, const double *px,
                                                    const double *py, const double *sgs, size_t n,
                                                    unsigned I, unsigned J, double *pu, double *pv,
@@ -286,11 +355,15 @@ __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, cons
                                                    sym::SourceBuffer &src) {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool diagonal = I == J;
-    const size_t ti = static_cast<size_t>(I) * kBlock + static_cast<size_t>(w) * 32 + lane;
-    const bool t_ok = ti < n;
     const auto vortex = [&](size_t i) {
         return i < n ? sym::Vortex{px[i], py[i], P::kScale * sgs[i]} : sym::Vortex{0.0, 0.0, 0.0};
     };
+    if (!diagonal) {
+        run_pair_item<P, T>(g, vortex, n, I, J, pu, pv, pad_n, red_u, red_v, src);
+        return;
+    }
+    const size_t ti = static_cast<size_t>(I) * kBlock + static_cast<size_t>(w) * 32 + lane;
+    const bool t_ok = ti < n;
     const sym::Vortex t = vortex(ti);
     double u = 0.0, v = 0.0;
     for (int qq = 0; qq < 4; ++qq) {
@@ -298,41 +371,11 @@ __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, cons
         const size_t sj = static_cast<size_t>(J) * kBlock + static_cast<size_t>(q) * 32 + lane;
         const int s_ok = sj < n ? 1 : 0;
         const sym::Vortex s = vortex(sj);
-        if (diagonal) {
-            sym::one_sided_tile<P>(g, t, t_ok, s, s_ok, q == w, u, v);
-        } else {
-            double ru = 0.0, rv = 0.0;
-            if (__all_sync(0xffffffffu, t_ok && s_ok)) {
-                const sym::Vortex t1[1] = {t};
-                double u1[1] = {u}, v1[1] = {v};
-                sym::react_tiles_full<P, 1, true>(g, t1, s, src, P::near(g, t.x, t.y), u1, v1, ru,
-                                                  rv);
-                u = u1[0];
-                v = v1[0];
-            } else {
-                sym::react_tile_t<P, false>(g, t, t_ok, s, s_ok, u, v, ru, rv);
-            }
-            red_u[w * kBlock + q * 32 + lane] = ru;
-            red_v[w * kBlock + q * 32 + lane] = rv;
-        }
+        sym::one_sided_tile<P>(g, t, t_ok, s, s_ok, q == w, u, v);
     }
     if (t_ok) {
         pu[static_cast<size_t>(J) * pad_n + ti] = u;
         pv[static_cast<size_t>(J) * pad_n + ti] = v;
-    }
-    if (!diagonal) {
-        __syncthreads();
-        const size_t sj = static_cast<size_t>(J) * kBlock + threadIdx.x;
-        if (sj < n) {
-            double su = red_u[threadIdx.x], sv = red_v[threadIdx.x];
-            for (int k = 1; k < 4; ++k) {
-                su += red_u[k * kBlock + threadIdx.x];
-                sv += red_v[k * kBlock + threadIdx.x];
-            }
-            pu[static_cast<size_t>(I) * pad_n + sj] = su;
-            pv[static_cast<size_t>(I) * pad_n + sj] = sv;
-        }
-        __syncthreads();
     }
 }
 
@@ -572,12 +615,11 @@ struct VelocityBatchArgs {
 };
 
 // PREC = PV_PRECISION_FP64: ordered and symmetric items; PREC = PV_PRECISION_FP32C: the
-// compensated form's ordered items. Built for 5 resident CTAs per SM: the FP64 form then holds
-// 96 registers (128 unbounded, 4 CTAs) without spills, and the 512-member mixed-N ensemble runs
-// 2 % faster in FP64 and 1 % in FP32C (six alternating runs, spread under 0.3 %); a bound of 6
-// spills the FP64 form and gains nothing.
+// compensated form's. FP64 is built for 4 resident CTAs per SM, whose 128 registers hold the pair items'
+// targets without spills (an attempt of the ensemble above 1.77 ms, for 5 CTAs with 104 bytes spilled
+// 1.87); FP32C for 5, which run its 512-member ensemble 1 % faster than 4.
 template <int PREC>
-__global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const VelocityBatchArgs a) {
+__global__ void __launch_bounds__(kBlock, PREC == PV_PRECISION_FP64 ? 4 : 5) batch_velocity_kernel(const VelocityBatchArgs a) {
     __shared__ alignas(128) double s_x[2][kTileB];
     __shared__ alignas(128) double s_y[2][kTileB];
     __shared__ alignas(128) double s_g[2][kTileB];
@@ -630,14 +672,17 @@ __global__ void __launch_bounds__(kBlock, 5) batch_velocity_kernel(const Velocit
             else {
                 sym::SourceBuffer &src = s_src[threadIdx.x >> 5];
                 if (s_geo.geometry == GEO_DISK)
-                    run_symmetric_item<sym::DiskSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu,
+                    run_symmetric_item<sym::DiskSym, 4>(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu,
                                                      pv, d.pad_n, &s_x[0][0], &s_y[0][0], src);
+                else if (s_geo.geometry == GEO_INFINITE)
+                    run_symmetric_item<sym::PlaneSym, 4>(s_geo, px, py, sgs, d.n, it.tb, it.chunk, pu,
+                                                         pv, d.pad_n, &s_x[0][0], &s_y[0][0], src);
                 else if (s_geo.zeta)
-                    run_symmetric_item<sym::ZetaUnitSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk,
+                    run_symmetric_item<sym::ZetaUnitSym, 2>(s_geo, px, py, sgs, d.n, it.tb, it.chunk,
                                                          pu, pv, d.pad_n, &s_x[0][0], &s_y[0][0],
                                                          src);
                 else
-                    run_symmetric_item<sym::PeriodicSym>(s_geo, px, py, sgs, d.n, it.tb, it.chunk,
+                    run_symmetric_item<sym::PeriodicSym, 1>(s_geo, px, py, sgs, d.n, it.tb, it.chunk,
                                                          pu, pv, d.pad_n, &s_x[0][0], &s_y[0][0],
                                                          src);
             }
@@ -1061,6 +1106,7 @@ pv_status rebuild_tables(pv_batch *b) {
         // a pair's cost in an item of its form: FP64 pipe cycles over the plane's ordered pair's 22
         const double w = d.g.geometry == GEO_PERIODIC ? (d.g.zeta && q == 0 ? 5.5 : 12.0)
                          : d.g.geometry == GEO_DISK   ? (d.symmetric ? 3.5 : 3.0)
+                         : d.symmetric                ? 1.4
                                                       : 1.0;
         if (d.symmetric) {
             const unsigned nb = symmetric_rows(d.n);
