@@ -321,9 +321,10 @@ pv_status pv_batch_status(pv_batch *batch, pv_batch_totals *totals);
 pv_status pv_batch_stream(const pv_batch *batch, void **stream);
 /* Autotuner table of the batch's ordered work items: targets per thread (1, 2 or 4; 4 not for the
  * periodic box; 0 restores the default of 4 for the plane, 1 for the box and 2 for the disk) for a
- * geometry, a precision and populations with floor(log2 N) == log2_n. FP64 box and disk members
- * of 128 to 4096 vortices take once-per-unordered-pair items where their size has no entry (0), and
- * ordered items where it has one. Process-wide; read when a simulation is admitted (pv_batch_add), so a simulation's work items, like its results, depend
+ * geometry, a precision and populations with floor(log2 N) == log2_n. FP64 members of 128 to 4096
+ * vortices take once-per-unordered-pair items where their size has no entry (0), and ordered items
+ * where it has one. Process-wide; read when a simulation is admitted (pv_batch_add), so a
+ * simulation's work items, like its results, depend
  * only on its own geometry, precision and N. pv_get_batch_tuning returns the value in effect. */
 pv_status pv_set_batch_tuning(int geometry, int precision, int log2_n, int per_thread);
 pv_status pv_get_batch_tuning(int geometry, int precision, int log2_n, int *per_thread);

@@ -9,8 +9,8 @@
 //     (simulation, block of 128 threads x T targets, chunk of sources) items with an atomic counter. The
 //     items are sorted by cost (a pair of the box costs 5-12 plane pairs), so the longest go first.
 //     Each CTA copies the item's geometry constants to shared memory and runs the same TMA-staged
-//     tile loop and pair functions as the single-simulation kernel. Periodic and disk simulations
-//     (batch_pair_items) instead take (simulation, block I, block J) items of 128 x 128 evaluated
+//     tile loop and pair functions as the single-simulation kernel. Simulations of the sizes of
+//     batch_pair_items() instead take (simulation, block I, block J) items of 128 x 128 evaluated
 //     once per unordered pair (the warp tiles of pv_symmetric.cuh, reactions summed across the
 //     CTA's warps in fixed order). Simulations in the FP32-compensated form drain a second queue, in a
 //     second launch, with the pair terms of pv_pair32.cuh;
@@ -98,7 +98,7 @@ bool batch_pair_items(const GeometryConsts &g, int precision, size_t n) {
         return true;
     if (precision != PV_PRECISION_FP64 || n > kPairRowsMaxN || batch_entry(g.geometry, precision, n) != 0)
         return false;
-    // the table of single simulations does not speak for the plane, whose rows it judges at their size
+    // the table of single simulations does not speak for the plane: it times them alone
     return g.geometry == GEO_INFINITE || (tuned == 0 && (g.geometry == GEO_DISK || g.zeta));
 }
 // Sources per work item, a function of the population only (so a simulation's summation order
