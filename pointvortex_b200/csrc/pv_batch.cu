@@ -277,13 +277,18 @@ __device__ __forceinline__ void run_item(const GeometryConsts &g, const double *
 
 // A 128 x 128 block pair (I < J), once per unordered pair: warp w holds T targets a lane, of share
 // w % H of block I's H = 4 / T, and meets H of block J's 32-source sub-tiles, from (w / H) H on. The T
-// warps of a share, and the H of a sub-tile, add up in fixed order.
+// warps of a share, and the H of a sub-tile, add up in fixed order, in rows of 128 of red_u and red_v: the
+// targets' T, then the reactions' H. With T = 1 a warp has its targets to itself, which then need no rows
+// and go straight to row J; with H = 1 it has its sources to itself.
+constexpr int kRedRows = 4;
 template <class P, int T, class Load>
 __device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Load &vortex, size_t n,
                                               unsigned I, unsigned J, double *pu, double *pv,
                                               size_t pad_n, double *red_u, double *red_v,
                                               sym::SourceBuffer &src) {
     constexpr int H = 4 / T;
+    constexpr int kTargetRows = T > 1 ? T : 0, kReactionRows = H > 1 ? H : 0;
+    static_assert(T * H == kBlock / 32 && kTargetRows + kReactionRows <= kRedRows);
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31, share = w % H, group = w / H;
     sym::Vortex t[T];
     bool t_ok[T], all_ok = true, near = true;
@@ -298,7 +303,8 @@ __device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Loa
         u[k] = v[k] = 0.0;
     }
 #pragma unroll 1
-    for (int q = H * group; q < H * group + H; ++q) {
+    for (int qq = 0; qq < H; ++qq) {
+        const int q = H * group + (T == 1 ? (w + qq) % H : qq);
         const size_t sj = static_cast<size_t>(J) * kBlock + static_cast<size_t>(q) * 32 + lane;
         const int s_ok = sj < n ? 1 : 0;
         const sym::Vortex s = vortex(sj);
@@ -311,8 +317,8 @@ __device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Loa
                 sym::react_tile_t<P, false>(g, t[k], t_ok[k], s, s_ok, u[k], v[k], ru, rv);
         }
         if (H > 1) {
-            red_u[(T + share) * kBlock + q * 32 + lane] = ru;
-            red_v[(T + share) * kBlock + q * 32 + lane] = rv;
+            red_u[(kTargetRows + share) * kBlock + q * 32 + lane] = ru;
+            red_v[(kTargetRows + share) * kBlock + q * 32 + lane] = rv;
         } else if (s_ok) {
             pu[static_cast<size_t>(I) * pad_n + sj] = ru;
             pv[static_cast<size_t>(I) * pad_n + sj] = rv;
@@ -320,8 +326,14 @@ __device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Loa
     }
 #pragma unroll
     for (int k = 0; k < T; ++k) {
-        red_u[group * kBlock + (share * T + k) * 32 + lane] = u[k];
-        red_v[group * kBlock + (share * T + k) * 32 + lane] = v[k];
+        if (T > 1) {
+            red_u[group * kBlock + (share * T + k) * 32 + lane] = u[k];
+            red_v[group * kBlock + (share * T + k) * 32 + lane] = v[k];
+        } else if (t_ok[k]) {
+            const size_t ti = static_cast<size_t>(I) * kBlock + share * 32 + lane;
+            pu[static_cast<size_t>(J) * pad_n + ti] = u[k];
+            pv[static_cast<size_t>(J) * pad_n + ti] = v[k];
+        }
     }
     __syncthreads();
     const auto add = [](const double *red, int rows) {
@@ -332,13 +344,13 @@ __device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Loa
     };
     const size_t ti = static_cast<size_t>(I) * kBlock + threadIdx.x;
     const size_t sj = static_cast<size_t>(J) * kBlock + threadIdx.x;
-    if (ti < n) {
+    if (T > 1 && ti < n) {
         pu[static_cast<size_t>(J) * pad_n + ti] = add(red_u, T);
         pv[static_cast<size_t>(J) * pad_n + ti] = add(red_v, T);
     }
     if (H > 1 && sj < n) {
-        pu[static_cast<size_t>(I) * pad_n + sj] = add(red_u + T * kBlock, H);
-        pv[static_cast<size_t>(I) * pad_n + sj] = add(red_v + T * kBlock, H);
+        pu[static_cast<size_t>(I) * pad_n + sj] = add(red_u + kTargetRows * kBlock, H);
+        pv[static_cast<size_t>(I) * pad_n + sj] = add(red_v + kTargetRows * kBlock, H);
     }
     __syncthreads();
 }
@@ -346,7 +358,7 @@ __device__ __forceinline__ void run_pair_item(const GeometryConsts &g, const Loa
 // One 128 x 128 block pair of an FP64 simulation, once per unordered pair by run_pair_item(). Targets'
 // sums go to row J, the sources' reactions to row I. A diagonal item (I == J) is evaluated one-sided:
 // warp w holds targets I*128 + 32w + lane and meets the four 32-source sub-tiles in turn. red_u / red_v:
-// 4 x 128 doubles of shared memory; src: the warp's source buffer.
+// kRedRows x 128 doubles of shared memory; src: the warp's source buffer.
 template <class P, int T>
 __device__ __forceinline__ void run_symmetric_item(const GeometryConsts &g, const double *px,
                                                    const double *py, const double *sgs, size_t n,
@@ -620,6 +632,7 @@ struct VelocityBatchArgs {
 // 1.87); FP32C for 5, which run its 512-member ensemble 1 % faster than 4.
 template <int PREC>
 __global__ void __launch_bounds__(kBlock, PREC == PV_PRECISION_FP64 ? 4 : 5) batch_velocity_kernel(const VelocityBatchArgs a) {
+    static_assert(2 * kTileB >= kRedRows * kBlock, "s_x and s_y are the pair items' red_u and red_v");
     __shared__ alignas(128) double s_x[2][kTileB];
     __shared__ alignas(128) double s_y[2][kTileB];
     __shared__ alignas(128) double s_g[2][kTileB];
