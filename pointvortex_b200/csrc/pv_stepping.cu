@@ -749,10 +749,18 @@ template <bool CLUSTER> struct StepShared {
         }
     }
 };
-size_t step_shared_bytes(size_t n, size_t targets, int chunks, bool cluster) {
+constexpr size_t step_shared_bytes(size_t n, size_t targets, size_t units, bool cluster) {
     const size_t np = (n + 1) & ~static_cast<size_t>(1);
-    return ((cluster ? 5 : 3) * np + 2 * targets * static_cast<size_t>(chunks) + 16 * targets) * sizeof(double);
+    return ((cluster ? 5 : 3) * np + 2 * units + 16 * targets) * sizeof(double);
 }
+// The most that small_steps_eligible() and small_steps_in_cluster() let a launch ask for.
+constexpr size_t step_shared_max(bool cluster) {
+    return cluster ? step_shared_bytes(kSmallStepsMaxN, (kSmallStepsMaxN + kClusterSteps - 1) / kClusterSteps,
+                                       kStepThreads, true)
+                   : step_shared_bytes(kSmallStepsMaxN, kStepThreads, kStepThreads * (kWideRows - 1), false);
+}
+static_assert(step_shared_max(false) <= 226 * 1024 && step_shared_max(true) <= 226 * 1024,
+              "a CTA's shared memory, with 1 KB to spare for the kernels' own");
 
 // One evaluation: positions (px, py) into shared memory (a cluster's are there), then the chunk sums of
 // the CTA's targets [t0, t0 + mine).
@@ -1027,12 +1035,16 @@ bool small_steps_eligible(size_t n, int num_chunks, int sm_count) {
 
 namespace {
 // The whole grid, one CTA per SM, cooperative (every CTA resident, or no launch at all), or one cluster.
+// The kernel's limit of shared memory belongs to the function, which the contexts of all host threads
+// launch: each sets it to the same value, the most any of them needs, since one that set its own launch's
+// size would take it from under another's.
 template <class Kernel>
 cudaError_t launch_steps(Kernel kernel, const SmallSteps &p, size_t grid, bool cluster,
                          cudaStream_t stream) {
-    const size_t smem = step_shared_bytes(p.n, (p.n + grid - 1) / grid, p.num_chunks, cluster);
+    const size_t targets = (p.n + grid - 1) / grid;
+    const size_t smem = step_shared_bytes(p.n, targets, targets * p.num_chunks, cluster);
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(smem));
+                                         static_cast<int>(step_shared_max(cluster)));
     if (e == cudaSuccess && cluster)
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess)
