@@ -325,9 +325,12 @@ pv_status pv_batch_stream(const pv_batch *batch, void **stream);
  * vortices take once-per-unordered-pair items where their size has no entry (0), and ordered items
  * where it has one. Process-wide; read when a simulation is admitted (pv_batch_add), so a
  * simulation's work items, like its results, depend
- * only on its own geometry, precision and N. pv_get_batch_tuning returns the value in effect. */
+ * only on its own geometry, precision and N. pv_get_batch_tuning returns the targets per thread that
+ * ordered items have (the default where there is no entry); pv_get_batch_tuning_entry the entry itself
+ * (0 where there is none), which is what to keep in order to put the table back. */
 pv_status pv_set_batch_tuning(int geometry, int precision, int log2_n, int per_thread);
 pv_status pv_get_batch_tuning(int geometry, int precision, int log2_n, int *per_thread);
+pv_status pv_get_batch_tuning_entry(int geometry, int precision, int log2_n, int *per_thread);
 
 /* ---- allocation-free evaluation (no counterpart in the reference) ------------------------ */
 

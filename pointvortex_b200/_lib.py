@@ -182,6 +182,7 @@ SIGNATURES = {
     "pv_get_symmetric_grid": (_ST, [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)]),
     "pv_set_batch_tuning": (_ST, [ctypes.c_int] * 4),
     "pv_get_batch_tuning": (_ST, [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)]),
+    "pv_get_batch_tuning_entry": (_ST, [ctypes.c_int] * 3 + [ctypes.POINTER(ctypes.c_int)]),
     "pv_set_profiling": (_ST, [_CTX, ctypes.c_int]),
     "pv_set_wait_limits": (_ST, [_CTX, ctypes.c_int64, ctypes.c_int64]),
     "pv_set_near_field": (_ST, [_CTX, ctypes.c_double]),

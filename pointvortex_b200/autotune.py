@@ -9,9 +9,10 @@ seeded state of that size, keeping the fastest in the library's tables:
   stage kernels, the captured attempt), the way the steppers use it;
 * for the chosen symmetric form, the persistent grid's CTAs per SM (pv_set_symmetric_grid): as
   many as fit, or down to three fewer (a fuller last round of the work queue can finish sooner);
-* the batch engine's ordered work items: 1, 2 or 4 targets per thread (pv_set_batch_tuning),
-  timed per DOPRI5 attempt of a batch of simulations of that size (as many as make about 2^26
-  pair interactions per evaluation, at most 512), so the choice is made where the grid is full.
+* the batch engine's work items: ordered ones with 1, 2 or 4 targets per thread
+  (pv_set_batch_tuning), or no entry, with which the sizes of its rule take once-per-unordered-pair
+  items. Timed per DOPRI5 attempt of a batch of simulations of that size (as many as make about
+  2^26 pair interactions per evaluation, at most 512), so the choice is made where the grid is full.
 
 Results are cached as JSON; the package loads `tuning.json` next to this file when it exists.
 
@@ -80,6 +81,14 @@ def set_batch_entry(geometry: int, precision: int, log2_n: int, per_thread: int)
 def get_batch_entry(geometry: int, precision: int, log2_n: int) -> int:
     out = ctypes.c_int(0)
     lib.pv_get_batch_tuning(geometry, precision, log2_n, ctypes.byref(out))
+    return out.value
+
+
+def stored_batch_entry(geometry: int, precision: int, log2_n: int) -> int:
+    """The entry itself, 0 where there is none (get_batch_entry reports the default there): what
+    set_batch_entry puts back."""
+    out = ctypes.c_int(0)
+    lib.pv_get_batch_tuning_entry(geometry, precision, log2_n, ctypes.byref(out))
     return out.value
 
 
@@ -222,11 +231,13 @@ def batch_room(n: int) -> tuple:
 
 def _time_batch(geometry: str, precision: str, n: int, attempts: int) -> float | None:
     """ms per DOPRI5 attempt of a batch of equal simulations of population n under the current
-    batch table, or None where the simulations take the once-per-unordered-pair items (the table
-    does not apply). Two untimed attempts first; the simulations run far from their end time."""
+    batch table, or None where the simulations take the once-per-unordered-pair items in spite of
+    an entry (the table does not apply). Two untimed attempts first; the simulations run far from
+    their end time."""
     import time
     from .batch import Batch, geometry_params
     sims, vortices, chunks = batch_room(n)
+    entry = stored_batch_entry(GEOMETRIES[geometry], PRECISIONS[precision], n.bit_length() - 1)
     b = Batch(vortices, sims, max_steps=1 << 30, partial_factor=chunks)
     try:
         for s in range(sims):
@@ -238,7 +249,7 @@ def _time_batch(geometry: str, precision: str, n: int, attempts: int) -> float |
                 st = ics.infinite_plane(n, 100 + s)
             sid = b.add(geometry_params(geometry, precision=precision), *st, 1e6, dt=1e-4,
                         atol=1e-10, rtol=1e-8)
-            if b.info(sid).targetsPerThread == 0:
+            if entry and b.info(sid).targetsPerThread == 0:
                 return None
         b.advance(2)
         t0 = time.perf_counter()
@@ -249,8 +260,9 @@ def _time_batch(geometry: str, precision: str, n: int, attempts: int) -> float |
 
 
 def tune_batch(log2_range=range(5, 16), attempts: int = 6) -> list:
-    """Each candidate of BATCH_CANDIDATES timed per attempt (_time_batch); the fastest is kept.
-    A size whose batch cannot be admitted (CapacityError: the device's memory) keeps the default
+    """Each candidate of BATCH_CANDIDATES and the built-in rule (no entry) timed per attempt
+    (_time_batch). The fastest candidate is kept, or no entry (per_thread 0) where the rule is
+    faster than all of them: the once-per-unordered-pair items are its choice only. A size whose batch cannot be admitted (CapacityError: the device's memory) keeps the default
     and is reported on stderr; the other sizes are still tuned."""
     import sys
     from .batch import CapacityError
@@ -275,9 +287,17 @@ def tune_batch(log2_range=range(5, 16), attempts: int = 6) -> list:
                     set_batch_entry(GEOMETRIES[geo], PRECISIONS[prec], b, 0)
                     continue
                 best = min(times, key=times.get)
+                set_batch_entry(GEOMETRIES[geo], PRECISIONS[prec], b, 0)
+                try:
+                    default_ms = _time_batch(geo, prec, 1 << b, attempts)
+                except CapacityError:  # its partial rows are more than the ordered items'
+                    default_ms = None
+                if default_ms is not None and default_ms < times[best]:
+                    best = 0
                 set_batch_entry(GEOMETRIES[geo], PRECISIONS[prec], b, best)
                 entries.append({"geometry": geo, "precision": prec, "log2_n": b, "per_thread": best,
-                                "ms": {str(k): v for k, v in times.items()}})
+                                "ms": {str(k): v for k, v in times.items()},
+                                "default_ms": default_ms})
     return entries
 
 

@@ -1577,6 +1577,14 @@ pv_status pv_get_batch_tuning(int geometry, int precision, int log2_n, int *per_
     return PV_OK;
 }
 
+pv_status pv_get_batch_tuning_entry(int geometry, int precision, int log2_n, int *per_thread) {
+    if (!per_thread || geometry < 0 || geometry > 2 || precision < 0 || precision > 1 ||
+        log2_n < 0 || log2_n >= 40)
+        return PV_ERROR_INVALID_ARGUMENT;
+    *per_thread = batch_entry(geometry, precision, size_t(1) << log2_n);
+    return PV_OK;
+}
+
 pv_status pv_batch_result(pv_batch *b, uint32_t id, double *x, double *y, size_t n) {
     if (!b || id >= b->max_sims || b->slot_used[id] == SIM_FREE)
         return PV_ERROR_INVALID_ARGUMENT;
