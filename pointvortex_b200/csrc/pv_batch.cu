@@ -99,7 +99,8 @@ bool batch_pair_items(const GeometryConsts &g, int precision, size_t n) {
     if (precision != PV_PRECISION_FP64 || n > kPairRowsMaxN || batch_entry(g.geometry, precision, n) != 0)
         return false;
     // the table of single simulations does not speak for the plane: it times them alone
-    return g.geometry == GEO_INFINITE || (tuned == 0 && (g.geometry == GEO_DISK || g.zeta));
+    return g.geometry == GEO_INFINITE ||
+           (tuned == 0 && (g.geometry == GEO_DISK ? disk_pairs_in_range(g) : g.zeta != 0));
 }
 // Sources per work item, a function of the population only (so a simulation's summation order
 // never depends on its batch): 512 up to N = 16384, then N/32 rounded up to 512.

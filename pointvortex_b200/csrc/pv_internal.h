@@ -98,6 +98,12 @@ constexpr size_t kSymmetricDiskMinN = 4096;
 // the disk from here 4 targets per lane, from half of it 2 (16 384: 314 against 326 us with 2;
 // 8192: 100 with 2 against 102 with 1; more per lane leaves too few items)
 constexpr size_t kSymmetricDiskWideN = 16384;
+// DiskSym squares R^2 - t.s, DiskPair 1 - t.s/R^2: for radii outside this range, where R^4 or the square near
+// the wall might not be a normal number, the disk keeps the ordered kernel. (Beyond R = 1e77 every pair of the
+// other would overflow and every target be recomputed one source after another.)
+inline bool disk_pairs_in_range(const GeometryConsts &g) {
+    return g.radius >= 0x1p-200 && g.radius <= 0x1p200;
+}
 constexpr size_t kSymmetricPartialBytes = static_cast<size_t>(256) << 20;  // a grows past this
 constexpr size_t kSymmetricPartialBytesMax = static_cast<size_t>(4) << 30;  // beyond: ordered kernel
 SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const GeometryConsts &g);

@@ -515,7 +515,7 @@ SymmetricPlan plan_symmetric(size_t n, int sm_count, int precision, const Geomet
     SymmetricPlan p{};
     const bool plane = geometry == GEO_INFINITE;
     const bool disk = geometry == GEO_DISK;
-    if (disk && precision == PV_PRECISION_FP32C)
+    if (disk && (precision == PV_PRECISION_FP32C || !disk_pairs_in_range(g)))
         return p;
     // the measured table overrides the built-in choice of form, occupancy and targets per lane
     const int tuned = symmetric_tuning_lookup(geometry, precision, n);
