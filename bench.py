@@ -462,8 +462,9 @@ def run_reference(args):
 def run_kernel_case(spec: str, evals: int, precision: str = "fp64", ordered: bool = False) -> dict:
     """Velocity evaluations only (no stepping), for kernel timing and ncu captures:
     spec = "geometry:N" with geometry infinite | periodic | disk; precision fp64 | fp32c.
-    ordered: evaluate host arrays (always the ordered-pair kernel) instead of the device state
-    (the symmetric kernel where the plan uses it)."""
+    ordered: evaluate all targets but the last of host arrays (fewer targets than vortices always
+    take the ordered-pair kernel) instead of the device state (the symmetric kernel where the plan
+    uses it)."""
     import torch
     import pointvortex_b200 as pv
     from pointvortex_b200 import ics
@@ -484,7 +485,9 @@ def run_kernel_case(spec: str, evals: int, precision: str = "fp64", ordered: boo
         flops, flops_sym = 33, 47
     k.uploadDeviceState(pv.VortexSystem(x, y, g))
     symmetric = k.statePlan()["symmetric"] and not ordered
-    run = (lambda: k.evaluate(x, y, g)) if ordered else k.evaluateDeviceState
+    targets = n - 1 if ordered else n
+    run = ((lambda: k.evaluateRange(x, y, g, None, 0, targets)) if ordered
+           else k.evaluateDeviceState)
     for _ in range(2):
         run()
     k.setProfiling(True)
@@ -495,7 +498,7 @@ def run_kernel_case(spec: str, evals: int, precision: str = "fp64", ordered: boo
     st = stats["velocity"]
     ms = st[2] / max(st[1], 1)
     near_ms = stats["near"][2] / max(stats["near"][1], 1) if stats["near"][1] else 0.0
-    pairs = n * (n - 1)
+    pairs = targets * (n - 1)
     work = (flops_sym * pairs / 2) if symmetric else flops * pairs
     torch.cuda.synchronize()
     return {"case": spec, "precision": precision, "kernel": "symmetric" if symmetric else "ordered",
@@ -949,7 +952,7 @@ def main(argv=None):
     ap.add_argument("--precision", choices=["fp64", "fp32c"], default="fp64",
                     help="precision form of --kernel-case")
     ap.add_argument("--ordered", action="store_true",
-                    help="--kernel-case on host arrays: the ordered-pair kernel")
+                    help="--kernel-case on a range of host arrays: the ordered-pair kernel")
     ap.add_argument("--reference-cuda", action="store_true",
                     help="time the reference's own CUDA backend on the workload (own process)")
     ap.add_argument("--summarize-launches", default=None, metavar="CSV",
