@@ -256,6 +256,11 @@ typedef struct pv_batch_config {
     uint64_t max_steps_per_simulation;     /* default accepted-step budget (0: unlimited) */
     size_t partial_chunks_per_vortex_slot; /* partial-sum room per arena vortex (0: 16) */
 } pv_batch_config;
+/* The arena takes 176 + 16 * partial_chunks_per_vortex_slot bytes a vortex, and 512 more for the partial
+ * sums of small members' once-per-unordered-pair items (FP64, 128 to 4096 vortices; pv_set_batch_tuning).
+ * A batch that fits into the device's free memory only without those 512 is made without them: such
+ * members then take ordered items (pv_batch_sim_info.targets_per_thread tells), whose sums are rounded in
+ * another order. */
 
 /* One solve: integrate to t_end with DOPRI5 (the reference driver's integrator dopri5). */
 typedef struct pv_batch_solve {

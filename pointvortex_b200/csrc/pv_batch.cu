@@ -87,16 +87,18 @@ int batch_targets_for(int geometry, int precision, size_t n) {
 //     full batches of one size, one target a lane (plane: ordered) and now, us: disk 24 x 4096 3572 and
 //     2998, box 5438 and 5040, plane 1894 and 1508, plane 300 x 256 392 and 338;
 //   * kPairRowsMaxN bounds the partial rows of these smaller members: kPairRows a vortex, which the
-//     arena holds beside the caller's own (pv_batch_create), so no admission is refused for them.
+//     arena holds beside the caller's own (pv_batch_create), so no admission is refused for them. A batch
+//     whose arena has no room for those rows (small_pairs false) leaves such members ordered items.
 constexpr size_t kPairRows = 32;
 constexpr size_t kPairRowsMaxN = kPairRows * 128;
-bool batch_pair_items(const GeometryConsts &g, int precision, size_t n) {
+bool batch_pair_items(const GeometryConsts &g, int precision, size_t n, bool small_pairs) {
     if (n < 128)
         return false;
     const int tuned = symmetric_tuning_lookup(g.geometry, precision, n) & 15;
     if (g.geometry == GEO_PERIODIC && (tuned == 2 || (tuned == 0 && n >= kSymmetricMinN)))
         return true;
-    if (precision != PV_PRECISION_FP64 || n > kPairRowsMaxN || batch_entry(g.geometry, precision, n) != 0)
+    if (!small_pairs || precision != PV_PRECISION_FP64 || n > kPairRowsMaxN ||
+        batch_entry(g.geometry, precision, n) != 0)
         return false;
     // the table of single simulations does not speak for the plane: it times them alone
     return g.geometry == GEO_INFINITE ||
@@ -998,6 +1000,7 @@ struct pv_batch {
     std::string error;
     size_t capacity = 0;        // vortices
     size_t part_capacity = 0;   // partial elements per array
+    bool small_pairs = true;    // ... with the rows of small members' pair items among them
     unsigned max_sims = 0;
     uint64_t default_max_steps = 0;
     Arena arena{};
@@ -1329,10 +1332,19 @@ pv_status pv_batch_create(const pv_batch_config *config, pv_batch **out) {
     // partials: each simulation needs ceil(n/512) chunks of pad(n); bounded by capacity^2/512 but
     // allocated as a multiple of the element capacity (sized by the caller's partial factor)
     const size_t factor = config->partial_chunks_per_vortex_slot ? config->partial_chunks_per_vortex_slot : 16;
-    b->part_capacity = b->capacity * (factor + kPairRows);
     const size_t arrays = 4 + 4 + 14;
-    const size_t bytes = (arrays * b->capacity + 2 * b->part_capacity) * sizeof(double);
-    if ((e = cudaMalloc(&b->arena_block, bytes)) != cudaSuccess)
+    const auto allocate = [&](size_t rows) {
+        b->part_capacity = b->capacity * rows;
+        return cudaMalloc(&b->arena_block,
+                          (arrays * b->capacity + 2 * b->part_capacity) * sizeof(double));
+    };
+    e = allocate(factor + kPairRows);
+    if (e == cudaErrorMemoryAllocation) {  // as large as the caller asked for, without those rows
+        cudaGetLastError();
+        b->small_pairs = false;
+        e = allocate(factor);
+    }
+    if (e != cudaSuccess)
         return bail(e, "cudaMalloc(batch arena)");
     double *p = static_cast<double *>(b->arena_block);
     auto next = [&](size_t n) {
@@ -1430,7 +1442,7 @@ pv_status pv_batch_add(pv_batch *b, const pv_params *params, const double *x, co
         return bfail(b, PV_ERROR_INVALID_ARGUMENT, "unknown precision form");
     const size_t pad = round_up(n, kAlign);
     const size_t chunk = chunk_for(n);
-    const bool symmetric = batch_pair_items(g, params->precision, n);
+    const bool symmetric = batch_pair_items(g, params->precision, n, b->small_pairs);
     const unsigned chunks = symmetric ? symmetric_rows(static_cast<unsigned>(n))
                                       : static_cast<unsigned>((n + chunk - 1) / chunk);
     size_t off = 0, poff = 0;
