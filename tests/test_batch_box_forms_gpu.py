@@ -23,8 +23,8 @@ MEMBERS = [(layers, length, n) for layers, length in ((1, TWO_PI), (3, TWO_PI), 
            for n in (2048, 2050, 4098)]
 
 
-def solve(members):
-    b = Batch(sum(n + 256 for _, _, n in members), len(members), max_steps=STEPS, partial_factor=64)
+def solve(members, steps=STEPS):
+    b = Batch(sum(n + 256 for _, _, n in members), len(members), max_steps=steps, partial_factor=64)
     ids = []
     for layers, length, n in members:
         unit = length / TWO_PI
@@ -67,16 +67,14 @@ def test_alone_in_the_mix_and_against_ordered_items(ordered_items):
         assert error <= 1e-14 * member[1] / TWO_PI, (member, error)
 
 
-@pytest.mark.parametrize("layers,n", [(1, 2048), (3, 2050), (5, 2050)])
+@pytest.mark.parametrize("layers,n", [(1, 2050), (5, 2048)])
 def test_matches_the_oracle(port, layers, n):
-    (info, (x, y)), = solve([(layers, TWO_PI, n)])
-    assert info.targetsPerThread == 0 and info.acceptedSteps == STEPS
+    (info, (x, y)), = solve([(layers, TWO_PI, n)], 1)
+    assert info.targetsPerThread == 0 and info.acceptedSteps == 1
     geo = Geometry("periodic", box_length_x=TWO_PI, box_length_y=TWO_PI, image_layers=layers,
                    absolute_tolerance=1e-10, relative_tolerance=1e-8, minimum_time_step=1e-6 * DT,
                    maximum_time_step=DT)
     xr, yr, g = ics.periodic_box(n, 3 + n, TWO_PI)
-    stepper = port.stepper(geo, n)
-    for _ in range(STEPS):
-        xr, yr, r = stepper.dopri5_step(xr, yr, g, DT)
-        assert r[0] == DT
+    xr, yr, r = port.stepper(geo, n).dopri5_step(xr, yr, g, DT)
+    assert r[0] == DT
     assert np.max(np.hypot(x - xr, y - yr)) <= 1e-14
