@@ -17,6 +17,7 @@
 // All combination arithmetic uses explicitly rounded operations (__dmul_rn/__dadd_rn/__ddiv_rn)
 // in the reference's order, so that given the same stage velocities the new state is bit-identical
 // to the reference's (which x86-64 g++ computes without FMA contraction).
+#include "pv_barrier.cuh"
 #include "pv_internal.h"
 
 #include <algorithm>
@@ -560,8 +561,8 @@ cudaError_t launch_stage(const StageArgs &a, cudaStream_t stream, int sm_count) 
 // 1024 192 -> 83.
 
 // Grid barrier over the CTAs of a cooperative launch. The arrival counter starts at zero (the control
-// block is reset before the launch) and only grows: the low 40 bits count arrivals, the r-th barrier
-// is open once they reach r * gridDim.x. One release-add per CTA, then polling with acquire loads.
+// block is reset before the launch): the r-th barrier is open once it has counted r * gridDim.x
+// (pv_barrier.cuh lays the word out). One release-add per CTA, then polling with acquire loads.
 //
 // A CTA that met an error in the phase adds it to its arrival, in one of two fields by the barrier's
 // parity; every CTA that passes the barrier sees it there and stops. (A CTA can be one barrier ahead
@@ -574,8 +575,6 @@ cudaError_t launch_stage(const StageArgs &a, cudaStream_t stream, int sm_count) 
 // the next one broken -- or it is broken and none does: later arrivals and pollers see the flag and
 // return. The breaker sets ST_TIMEOUT. Since the state is written only in phases that follow an
 // open barrier, a timeout leaves it at the last completed step.
-constexpr unsigned long long kBarrierCount = (1ull << 40) - 1;
-// errors: 11 bits each from bit 40 and from bit 51, so at most 2047 CTAs
 struct GridBarrier {
     unsigned long long *arrivals;
     int *status;
@@ -591,12 +590,11 @@ struct GridBarrier {
     __device__ __forceinline__ bool wait(bool bad) {
         __shared__ int go;
         const int any_bad = __syncthreads_or(bad);
-        open_at += gridDim.x;
+        open_at += barrier::arrivals(gridDim.x);
         parity ^= 1u;
         if (threadIdx.x == 0) {
-            const int shift = parity ? 51 : 40;
-            const unsigned long long broken = parity ? 1ull << 63 : 1ull << 62;
-            const unsigned long long mine = 1ull + (any_bad ? 1ull << shift : 0ull);
+            const unsigned long long broken = barrier::broken(parity);
+            const unsigned long long mine = barrier::arrival(any_bad != 0, parity);
             // this CTA's writes, ordered by the __syncthreads, before its arrival
             asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(arrivals), "l"(mine)
                          : "memory");
@@ -608,7 +606,7 @@ struct GridBarrier {
                     ok = 0;
                     break;
                 }
-                if ((now & kBarrierCount) >= open_at)
+                if (barrier::open(now, open_at))
                     break;
                 if (it >= limit) {
                     const unsigned long long seen = atomicCAS(arrivals, now, now | broken);
@@ -628,7 +626,7 @@ struct GridBarrier {
                              : "l"(arrivals)
                              : "memory");
             }
-            if (ok && ((now >> shift) & 0x7ffull))
+            if (ok && barrier::errors(now, parity))
                 ok = 0;
             go = ok;
         }
@@ -1030,7 +1028,7 @@ bool small_steps_in_cluster(const GeometryConsts &g, size_t n, int num_chunks) {
 bool small_steps_eligible(size_t n, int num_chunks, int sm_count) {
     const size_t grid = static_cast<size_t>(sm_count > 0 ? sm_count : 148);
     return n >= 1 && n <= kSmallStepsMaxN && num_chunks >= 1 && num_chunks < kWideRows &&
-           grid <= 2047 && (n + grid - 1) / grid <= kStepThreads;
+           grid <= barrier::kMaxCtas && (n + grid - 1) / grid <= kStepThreads;
 }
 
 namespace {
