@@ -1,7 +1,8 @@
 """Autotuner of the velocity plans, per geometry, precision and N bucket (floor(log2 N)), on a
 seeded state of that size, keeping the fastest in the library's tables:
 
-* the ordered-pair kernel: 1, 2 or 4 targets per thread (pv_set_tuning);
+* the ordered-pair kernel: 1, 2 or 4 targets per thread (pv_set_tuning), timed per launch on all
+  targets but one, which is never the once-per-unordered-pair form;
 * the once-per-unordered-pair form of the periodic box and the plane (pv_set_symmetric_tuning):
   the ordered kernel or the symmetric form, and for the symmetric form the occupancy it is built
   for (periodic FP64: the default, 7 or 8 CTAs per SM) or the targets per lane (plane: 4 or 8).
@@ -112,7 +113,9 @@ def load(path: str = DEFAULT_PATH) -> int:
 
 
 def _time_plan(geometry: str, precision: int, n: int, per_thread: int, evals: int) -> float:
-    from .kernel import DiskKernel, InfinitePlaneKernel, PeriodicBoxKernel, VortexSystem
+    """ms of a launch of the ordered-pair kernel, on all targets but the last of a population of n:
+    the evaluation of all of them takes the once-per-unordered-pair form where that is planned."""
+    from .kernel import DiskKernel, InfinitePlaneKernel, PeriodicBoxKernel
     set_entry(GEOMETRIES[geometry], precision, n.bit_length() - 1, per_thread)
     if geometry == "infinite":
         k = InfinitePlaneKernel(0.0, precision=precision)
@@ -123,12 +126,11 @@ def _time_plan(geometry: str, precision: int, n: int, per_thread: int, evals: in
     else:
         k = DiskKernel(1.0, precision=precision)
         x, y, g = ics.disk(n, 1)
-    k.uploadDeviceState(VortexSystem(x, y, g))
-    k.evaluateDeviceState()
+    k.evaluateRange(x, y, g, None, 0, n - 1)
     k.setProfiling(True)
     k.resetKernelStats()
     for _ in range(evals):
-        k.evaluateDeviceState()
+        k.evaluateRange(x, y, g, None, 0, n - 1)
     _, timed, ms = k.kernelStats()["velocity"]
     k.close()
     return ms / max(timed, 1)
