@@ -65,8 +65,12 @@ class Completion:
     engine: str = "batch"         # batch: in a batched launch; context: alone on a context
 
 
-# Relative cost of one ordered pair by geometry, from the measured FP64 pair rates of the
-# single-simulation kernels (plane 1.5e12, disk 5.3e11, periodic 9.6e10 pairs/s).
+# Weights of one ordered pair by geometry for the choice of a lane and for shortest-first order, which
+# split_work goes with: pair rates of the FP64 ordered kernels (plane 1.5e12, disk 5.3e11) and of the
+# box's image sums (9.6e10 pairs/s), under which box requests above N = 2061 count as expensive. The
+# kernels' rates have since drawn together (N = 16384: 1.8e12, 8.4e11 and 5.4e11). With weights of those,
+# 2.1 and 3.3, box requests up to N = 4500 join the cheap lane, and at 30 requests a second the policy
+# "split" answers at a median of 4 to 8 ms instead of 3; other rates and "split_context" stay as they are.
 PAIR_COST = {"infinite": 1.0, "disk": 2.9, "periodic": 15.8}
 
 
