@@ -172,13 +172,23 @@ SYMMETRIC_CANDIDATES = {
 }
 
 
+# Populations up to this take whole steps in one launch where the ordered kernel is asked for.
+SMALL_STEPS_MAX_N = 2048
+
+
+def symmetric_size(b: int) -> int:
+    """The population that stands for bucket b in tune_symmetric: 2^b, or the bucket's middle where 2^b
+    is one that small steps serve, which say nothing of the larger ones."""
+    return 1 << b if 1 << b > SMALL_STEPS_MAX_N else 3 << (b - 1)
+
+
 def tune_symmetric(log2_range=range(11, 17), evals: int = 3) -> list:
     """Each candidate timed per evaluation inside DOPRI5 steps (_time_steps), 3 + evals steps."""
     entries = []
     steps = max(evals, 3)
     for (geo, prec), cands in SYMMETRIC_CANDIDATES.items():
         for b in log2_range:
-            n = 1 << b
+            n = symmetric_size(b)
             times = {}
             for cand in cands:
                 set_symmetric_entry(GEOMETRIES[geo], PRECISIONS[prec], b, *cand)
@@ -196,7 +206,7 @@ def tune_symmetric(log2_range=range(11, 17), evals: int = 3) -> list:
                 best_c = min(grid_ms, key=grid_ms.get)
                 grid = 0 if best_c == fit else best_c
             set_symmetric_grid(GEOMETRIES[geo], PRECISIONS[prec], b, grid)
-            entries.append({"geometry": geo, "precision": prec, "log2_n": b, "mode": best[0],
+            entries.append({"geometry": geo, "precision": prec, "log2_n": b, "n": n, "mode": best[0],
                             "min_ctas": best[1], "targets": best[2], "grid_ctas": grid,
                             "ms": {"/".join(map(str, c)): v for c, v in times.items()},
                             "grid_ms": {str(c): v for c, v in grid_ms.items()}})
