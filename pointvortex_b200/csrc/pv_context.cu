@@ -113,6 +113,7 @@ struct pv_context {
     };
     PairItems sym_items;             // the device state's
     PairItems eval_items;            // host evaluations'
+    size_t eval_rows_refused = SIZE_MAX;  // doubles of their rows that the device had no memory for
     DeviceArray inv_scratch, inv_out;
     DeviceArray cand;                // dipole candidates (3 doubles-worth each)
     char *stage = nullptr;           // pinned staging, its size, and whether uploads may still read it
@@ -778,13 +779,19 @@ pv_status evaluate_host(pv_context *c, const double *x, const double *y, const d
     // upload and first evaluation differ from this in nothing (whole calls, ordered and so: box N = 2048
     // 107 and 93 us, 12 000 657 and 398; disk 4096 114 and 112, 12 000 422 and 300; plane 16 400 373 and
     // 341, 24 000 623 and 498). Rows that do
-    // not fit into the memory left, which the chunks' partials may, leave the ordered form.
+    // not fit into the memory left, which the chunks' partials may, leave the ordered form, also of later
+    // calls: asking again each time, with the chunks' partials given back and taken, adds 1 ms to a call of
+    // 15.5 (N = 65 536, ordered), and 100 now and then.
     SymmetricPlan sym{};
     if (nt == n && c->params.precision == PV_PRECISION_FP64)
         sym = plan_symmetric(n, c->sm_count, c->params.precision, c->gc);
-    if (sym.enabled() && (c->epu.ensure(2 * static_cast<size_t>(sym.blocks) * stride) != cudaSuccess ||
+    const size_t rows = 2 * static_cast<size_t>(sym.blocks) * stride;
+    if (rows >= c->eval_rows_refused)
+        sym = SymmetricPlan{};
+    if (sym.enabled() && (c->epu.ensure(rows) != cudaSuccess ||
                           ensure_pair_items(c, c->eval_items, sym) != cudaSuccess)) {
         cudaGetLastError();
+        c->eval_rows_refused = rows;
         sym = SymmetricPlan{};
     }
     if (!sym.enabled()) {
