@@ -736,14 +736,20 @@ pv_status ensure_state_capacity(pv_context *c, size_t n) {
         if (st != PV_OK)
             return st;
     }
-    const size_t rows = c->sym.enabled() ? static_cast<size_t>(c->sym.blocks)
-                                         : static_cast<size_t>(c->plan.num_chunks);
-    const size_t partial = rows * np;
-    // the symmetric kernels' rows hold (u, v) pairs in pu's room; the chunk partials use both
-    PV_CUDA(c, c->pu.ensure(c->sym.enabled() ? 2 * partial : partial));
-    PV_CUDA(c, c->pv.ensure(c->sym.enabled() ? 1 : partial));
-    if (c->sym.enabled())
-        PV_CUDA(c, ensure_pair_items(c, c->sym_items, c->sym));
+    // the symmetric kernels' rows hold (u, v) pairs in pu's room; the chunk partials use both. Rows that do
+    // not fit into the memory left, which the chunks' partials may (N = 65 536: 256 and below 64 MB), leave the
+    // ordered form.
+    if (c->sym.enabled() &&
+        (c->pu.ensure(2 * static_cast<size_t>(c->sym.blocks) * np) != cudaSuccess ||
+         c->pv.ensure(1) != cudaSuccess || ensure_pair_items(c, c->sym_items, c->sym) != cudaSuccess)) {
+        cudaGetLastError();
+        c->sym = SymmetricPlan{};
+    }
+    if (!c->sym.enabled()) {
+        const size_t partial = static_cast<size_t>(c->plan.num_chunks) * np;
+        PV_CUDA(c, c->pu.ensure(partial));
+        PV_CUDA(c, c->pv.ensure(partial));
+    }
     return PV_OK;
 }
 
