@@ -379,7 +379,7 @@ typedef struct pv_kernel_stats {
 /* The context's CUDA stream (a cudaStream_t) through *stream, so that a caller can order its own
  * work or events after the context's kernels. */
 pv_status pv_context_stream(const pv_context *ctx, void **stream);
-/* Autotuner table of the velocity plan: targets held in registers per thread (1, 2 or 4; 0 restores
+/* Autotuner table of the ordered kernel's plan: targets held in registers per thread (1, 2 or 4; 0 restores
  * the built-in heuristic) for a geometry, a precision and populations N with floor(log2 N) ==
  * log2_n. Process-wide; read when a context plans an evaluation (pv_upload_state,
  * pv_evaluate_range). pointvortex_b200/autotune.py fills it by timing the candidates. */
@@ -414,7 +414,8 @@ pv_status pv_set_near_field(pv_context *ctx, double radius);
 pv_status pv_get_near_field(const pv_context *ctx, double *radius);
 /* Polls of the context's bounded device waits before they give up with the runtime error "a bounded
  * device wait timed out": copy_polls for a velocity tile's bulk copies (default 2^22), barrier_polls
- * for a grid barrier of the cooperative RK4 steps (default 2^24); a negative value restores the
+ * for a grid barrier of the cooperative steps (default 2^24; a context that sets it does not take the
+ * cluster form of the smallest steps, whose barrier has no limit); a negative value restores the
  * default, 0 gives up without polling. A wait that gives up leaves the device state at the last
  * completed step (a velocity tile first waits, with the default bound, for its copies in flight; a
  * grid barrier is broken for every CTA at once). Only the tests of these exits shorten them. No

@@ -1,5 +1,5 @@
 // pv_symmetric.cu — the velocity of a whole population evaluated once per unordered pair: the
-// periodic box and the infinite plane, each in FP64 and in the FP32-compensated form.
+// periodic box and the infinite plane, each in FP64 and in the FP32-compensated form, and the FP64 disk.
 //
 // The reference evaluates every ordered pair (src/compute.cpp:203-256 for the box, :88-133 for
 // the plane). The Weiss–McWilliams pair term is antisymmetric: exchanging target and source
@@ -7,18 +7,20 @@
 // an exactly odd or even function of them, so the source's term is the target's with the other
 // circulation and the opposite sign, bit for bit. The plane's (dy, dx) / (r^2 + eps^2) is odd in
 // the same way. One evaluation therefore serves both vortices, and the work per velocity
-// evaluation halves. Only the order of summation differs from the ordered-pair kernel.
+// evaluation halves. Only the order of summation differs from the ordered-pair kernel. The disk's image
+// term is not antisymmetric, but its reciprocal serves both vortices (sym::DiskSym).
 //
 // Work decomposition (warp-level, persistent):
 //   * vortices form blocks of 32a (a = 1..16 sub-blocks of 32); an item is a block pair (I, J),
 //     I <= J, taken by one warp from an atomic queue;
-//   * for a sub-block pair each lane holds one target; the 32 sources and their accumulated
-//     reactions rotate through the lanes by shuffles, so in 32 steps every (target, source) pair
-//     is met once and every source comes back to its home lane;
+//   * for a sub-block pair each lane holds one target and reads the 32 sources from the warp's shared
+//     buffer, a different one each step; the reactions that they accumulate rotate through the lanes by
+//     shuffles, so in 32 steps every (target, source) pair is met once and every reaction comes back to
+//     its home lane;
 //   * sub-blocks on the diagonal of a diagonal item are evaluated one-sided (31 rotations, the
-//     self pair skipped, as in the reference);
-//   * the plane's pair term is cheap next to the five shuffles of a rotation step, so off the
-//     diagonal each lane holds 4 or 8 targets against the rotating sources;
+//     self pair skipped, as in the reference; the disk's image of a vortex itself added);
+//   * off the diagonal each lane holds more targets where that pays, which share a step's shuffles: the
+//     plane 4 or 8 (with 8 the sources rotate too), the disk 1, 2 or 4 and the box 1 or 2;
 //   * partial sums go to rows of a [blocks][N] array of (u, v) pairs (one 16-byte store per entry):
 //     vortices of block I receive row J from item (I, J), vortices of block J receive row I, and
 //     each (row, vortex) is written exactly once, so the stage kernel's fixed-order sum over rows
@@ -51,7 +53,7 @@ __device__ __forceinline__ void release_queue(unsigned *counter) {
     }
 }
 
-// P: the pair kernel (sym::PeriodicSym, sym::PlaneSym). T: targets per lane in the items off the
+// P: the pair kernel (sym::PeriodicSym, sym::ZetaSym, sym::PlaneSym, sym::DiskSym). T: targets per lane in the items off the
 // diagonal (a multiple of T sub-blocks per block); diagonal items hold one target per lane.
 // MINB: resident CTAs per SM the register allocation must allow (0: the compiler's own choice;
 // the periodic kernel is also built for 7 and 8, fewer registers for more warps to hide latency).
